@@ -136,12 +136,12 @@ int brc_ctx::tune_tc(int nfilt, int W, int H, int D, const uint16_t* d_taps, boo
 
 int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const float* fx, const float* fy,
                     const float* fz, const float* cert, const float* scert, float* tmp1, float* tmp2, float* out,
-                    cudaStream_t st, int accumulate, float* tune_out) {
-  const auto key = std::make_tuple(W, H, D, batch, (cert ? 1 : 0) + (scert ? 2 : 0));
+                    cudaStream_t st, int accumulate, float* tune_out, bool times_cert) {
+  const auto key = std::make_tuple(W, H, D, batch, (cert ? 1 : 0) + (scert ? 2 : 0) + (times_cert ? 4 : 0));
   auto it = smooth_tuned.find(key);
   if (it != smooth_tuned.end()) {
     BRC_TRY(this, brc::smooth3d(vol, W, H, D, batch, fx, fy, fz, cert, scert, tmp1, tmp2, out, st, accumulate,
-                                it->second),
+                                it->second, times_cert),
             "smooth3d");
     return BRC_OK;
   }
@@ -161,7 +161,8 @@ int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const floa
   int cand[8];
   const int n = brc::smooth3d_chunk_candidates(D, cand, 8);
   if (alias || cap != cudaStreamCaptureStatusNone || n < 2) {
-    BRC_TRY(this, brc::smooth3d(vol, W, H, D, batch, fx, fy, fz, cert, scert, tmp1, tmp2, out, st, accumulate),
+    BRC_TRY(this, brc::smooth3d(vol, W, H, D, batch, fx, fy, fz, cert, scert, tmp1, tmp2, out, st, accumulate, 0,
+                                times_cert),
             "smooth3d");
     return BRC_OK;
   }
@@ -179,7 +180,8 @@ int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const floa
     for (int rep = 0; rep < 3 && err == cudaSuccess; rep++) {
       err = cudaEventRecord(e0, st);
       if (err == cudaSuccess)
-        err = brc::smooth3d(vol, W, H, D, batch, fx, fy, fz, cert, scert, tmp1, tmp2, dst, st, 0, cand[c]);
+        err = brc::smooth3d(vol, W, H, D, batch, fx, fy, fz, cert, scert, tmp1, tmp2, dst, st, 0, cand[c],
+                            times_cert);
       if (err == cudaSuccess) err = cudaEventRecord(e1, st);
       if (err == cudaSuccess) err = cudaEventSynchronize(e1);
       float ms = 0.f;
@@ -531,15 +533,14 @@ int brc_smooth_normalized(brc_ctx* ctx, const float* d_vols, int W, int H, int D
   BRC_TRY(ctx, ctx->smask.ensure(sizeof(float) * (size_t)V), "alloc");
   const cudaStream_t st = ctx->stream();
   // smoothed certainty (all-ones certainty), then the certainty-weighted
-  // smoothing of every volume divided by it, then the mask product
+  // smoothing of every volume, divided by it and multiplied by the mask
   int s = ctx->smooth(d_mask, W, H, D, 1, h_fx, h_fy, h_fz, nullptr, nullptr, ctx->tmp1.as<float>(),
                       ctx->tmp2.as<float>(), ctx->smask.as<float>(), st);
   if (s != BRC_OK) return s;
   s = ctx->smooth(d_vols, W, H, D, T, h_fx, h_fy, h_fz, d_mask, ctx->smask.as<float>(), ctx->tmp1.as<float>(),
-                  ctx->tmp2.as<float>(), d_out, st);
+                  ctx->tmp2.as<float>(), d_out, st, 0, nullptr, true);
   if (s != BRC_OK) return s;
-  BRC_TRY(ctx, brc::multiply_mask(d_out, d_mask, V, T, st), "multiply mask");
-  ctx->launches += 3;
+  ctx->launches += 2;
   return BRC_OK;
 }
 

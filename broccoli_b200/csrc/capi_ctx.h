@@ -139,7 +139,7 @@ struct brc_ctx {
   // untimed choice.
   int smooth(const float* vol, int W, int H, int D, int batch, const float* fx, const float* fy, const float* fz,
              const float* cert, const float* scert, float* tmp1, float* tmp2, float* out, cudaStream_t st,
-             int accumulate = 0, float* tune_out = nullptr);
+             int accumulate = 0, float* tune_out = nullptr, bool times_cert = false);
 
   size_t workspace() const {
     return q1.bytes + q2.bytes + aligned.bytes + partials.bytes + ctl.bytes + tmp1.bytes +

@@ -57,10 +57,13 @@ cudaError_t warp_field(const float* src, int W, int H, int D, const float* dx, c
 cudaError_t rescale_linear(const float* src, int W, int H, int D, float* out, int W2, int H2, int D2,
                            cudaStream_t st);
 // zchunk: planes per z chunk of a CTA (0: the untimed choice
-// smooth3d_default_chunk); every choice gives the same result.
+// smooth3d_default_chunk); every choice gives the same result.  times_cert:
+// the quotient is multiplied by the certainty (needs cert and scert, no
+// accumulation).
 cudaError_t smooth3d(const float* vol, int W, int H, int D, int batch, const float* fx,
                      const float* fy, const float* fz, const float* cert, const float* scert,
-                     float* tmp1, float* tmp2, float* out, cudaStream_t st, int accumulate = 0, int zchunk = 0);
+                     float* tmp1, float* tmp2, float* out, cudaStream_t st, int accumulate = 0, int zchunk = 0,
+                     bool times_cert = false);
 int smooth3d_default_chunk(int W, int H, int D, int batch);
 int smooth3d_chunk_candidates(int D, int* zc, int max_n);
 // out[i] = phase_atan2(y[i], x[i]) (the arctangent of the phase kernels).

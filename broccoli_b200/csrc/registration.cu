@@ -881,10 +881,6 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
 // Separable 9-tap smoothing (three passes)
 // ---------------------------------------------------------------------------
 
-struct Taps9 {
-  float f[9];
-};
-
 // The three separable 9-tap passes in one kernel: y over (vol * cert), then
 // x, then z, divided by the smoothed certainty (SeparableConvolutionRows /
 // Columns / Rods, kernelConvolution.cpp:52-91, :531-569, :1201-1240, zero
@@ -892,222 +888,263 @@ struct Taps9 {
 // passes (o = -4..4 in order, out-of-volume terms 0), and the volume is read
 // from HBM once and written once.
 //
-// A block owns a 56 x 16 column tile and marches along z through a chunk of
-// planes.  Per plane, the 64 x 24 input window (tile plus 4-voxel halo) is
-// copied into shared memory with cp.async (zero-filled outside the volume)
-// into a four-stage ring, three planes ahead of its use; with an even W the
-// copies move 8-byte pairs (a pair never straddles the volume's edge), and a
-// thread's copies lie in one window column, so its addresses advance by a
-// constant.  Every thread then computes four y outputs of one window column
-// (12 shared loads, 36 FMAs), and 224 of the 256 threads four consecutive x
-// outputs of one tile row (three 16-byte shared loads, 36 FMAs), which enter
-// a nine-plane register ring; the z pass (36 FMAs) writes the output plane
-// to shared memory, from which all threads store it coalesced in the next
-// phase.  The ring slot of a plane is its index modulo 9, dispatched by a
-// switch over nine copies of the z pass so that every register index is a
-// constant.  The y pass of plane k, the x and z passes of plane k - 1 and
-// the stores of plane k - 2 run in the same phase (the y results and the
-// output plane are double-buffered), so one barrier per plane separates
-// every producer from its consumer.  With a certainty, its window is copied
-// beside the volume's and the product is formed in the y pass.  `out` must
-// not overlap the inputs.
-constexpr int kSmTX = 56, kSmTY = 16;            // output tile
-constexpr int kSmWX = kSmTX + 8, kSmWY = kSmTY + 8;  // input window 64 x 24
-constexpr int kSmPitch = 68;                     // shared row pitch (floats, 16-byte rows)
-constexpr int kSmThreads = 256;
-constexpr int kSmXQ = kSmTX / 4;                 // 14 quads of x outputs per row
-constexpr int kSmOwners = kSmXQ * kSmTY;         // 224 threads own outputs
-constexpr int kSmStages = 4;                     // window ring (planes in flight + 1)
-constexpr int kSmWin = kSmWY * kSmPitch;         // floats per window stage
-constexpr int kSmYBuf = kSmTY * kSmPitch;        // floats per y-result buffer
-constexpr int kSmOut = kSmTY * kSmTX;            // floats per output plane
-static_assert(kSmWX == 64 && kSmTY == 16, "mappings assume 64 window columns and 16 tile rows");
+// A block owns a column tile of up to 64 x 8 outputs and marches along z
+// through a chunk of planes, eight planes (a group) at a time:
+//   y  a thread takes one pair of window columns of a plane: sixteen 8-byte
+//      loads straight from global memory, 72 packed FMAs, eight 8-byte stores
+//      to the shared y buffer;
+//   x  a thread takes eight consecutive outputs of a row: four 16-byte
+//      shared loads, 36 packed FMAs on aligned and shifted pairs, two 16-byte
+//      stores into a ring of sixteen planes.  Its lanes run along the rows,
+//      whose pitches (12 and 4 modulo 32 banks) keep the 16-byte accesses
+//      free of conflicts;
+//   z  a thread takes one column pair: sixteen 8-byte loads from the ring, the
+//      eight output planes of the group in 72 packed FMAs, stored coalesced.
+// The z pass of a group runs in the same interval as the y pass of the next,
+// so a group has two barriers.  What a thread works on is decoded once: the
+// groups differ only by the plane offset.  This layout is for instruction
+// issue, which bounds the kernel: a form with a shared-memory window per
+// plane and a register ring for z issued 109 thread instructions per voxel
+// for its 27 FMAs.  Packed FP32 FMAs (two lanes per instruction, rounded as
+// two scalar ones) halve the issue slots of the arithmetic.
+// Measured (CUDA events): 9 volumes of 182x218x182 278 -> 174 us (3.0 TB/s),
+// 9 of 91x109x91 (odd width) 59 -> 37 us, 200 of 64x64x33 175 -> 73 us (3.0
+// TB/s), the same with certainty, division and mask product in the kernel
+// 360 -> 173 us.  Issue is now 63 % and the FMA pipe 46 % of the cycles
+// (warps wait at the group's barriers and for the window's loads).
+// `out` must not overlap the inputs.
+constexpr int kSmTX = 64, kSmTY = 8;    // largest output tile (the width is chosen per volume)
+constexpr int kSmG = 8;                 // planes per group
+constexpr int kSmThreads = 288;         // y units of a 64-wide tile: 36 column pairs x 8 planes
+constexpr int kSmPY = kSmTX + 12;       // y buffer pitch: 76 floats, 12 modulo 32
+constexpr int kSmPR = kSmTX + 4;        // ring pitch: 68 floats, 4 modulo 32
+constexpr int kSmYPlane = kSmTY * kSmPY, kSmRPlane = kSmTY * kSmPR;
+constexpr int kSmRGroup = kSmG * kSmRPlane;
+constexpr size_t kSmSmem = sizeof(float) * (kSmG * kSmYPlane + 2 * kSmRGroup);
+static_assert(kSmTY == 8 && kSmG == 8, "the unit decodes assume 8 rows and groups of 8 planes");
 
-inline size_t smooth_smem_bytes(bool cert) {
-  return sizeof(float) * ((size_t)(cert ? 2 : 1) * kSmStages * kSmWin + 2 * kSmYBuf + 2 * kSmOut);
+// Two floats in one 64-bit register, and the packed operations on them; each
+// lane rounds as the scalar instruction does.
+typedef unsigned long long F2;
+__host__ __device__ __forceinline__ F2 f2_twice(float v) {
+  union {
+    float f[2];
+    F2 u;
+  } r;
+  r.f[0] = r.f[1] = v;
+  return r.u;
+}
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
-template <int BYTES>
-__device__ __forceinline__ void cp_async(uint32_t dst, const float* src, uint32_t n) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"(BYTES), "r"(n)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// The taps of the three passes, each twice (both lanes of a packed FMA), in
+// the order of the samples (o = -4..4 meets taps 8..0).
+struct SmoothTaps {
+  F2 x[9], y[9], z[9];
+};
+
+// Output width of a block's tile: W in equal parts of at most 64, rounded up to
+// whole octets of the x pass.
+__host__ __device__ inline int smooth_tile_width(int W) {
+  const int n = (W + kSmTX - 1) / kSmTX;
+  return ((W + n - 1) / n + 7) / 8 * 8;
 }
 
-// VEC: floats per copy (2 needs an even W and 8-byte aligned volumes); DIV:
-// divide by the smoothed certainty scert; ACC: add into `out`.
-template <bool CERT, int VEC, bool DIV, bool ACC>
-__global__ void __launch_bounds__(kSmThreads, 3)
-smooth3d_kernel(const float* __restrict__ in, long long in_stride, const float* __restrict__ cert,
-                const float* __restrict__ scert, int W, int H, int D, int zc, Taps9 tx, Taps9 ty, Taps9 tz,
-                float* __restrict__ out, long long out_stride) {
+// VEC: pairs move as 8 bytes (an even W, so that no pair straddles the edge,
+// and 8-byte aligned volumes); DIV: divide by the smoothed certainty scert;
+// MUL: then multiply by the certainty; ACC: add into `out`.
+template <bool CERT, bool VEC, bool DIV, bool MUL, bool ACC>
+// Three blocks per SM (72 registers) where pairs move and there is no
+// certainty; the other forms spill there and run faster with two (odd width, 9
+// volumes of 91x109x91: 37 against 49 us; certainty, 200 volumes of 64x64x33:
+// 173 against 175 us).
+__global__ void __launch_bounds__(kSmThreads, VEC && !CERT ? 3 : 2)
+smooth3d_kernel(const float* __restrict__ in, const float* __restrict__ cert, const float* __restrict__ scert,
+                int W, int H, int D, int tw, int zc, const __grid_constant__ SmoothTaps taps,
+                float* __restrict__ out) {
   extern __shared__ __align__(16) float smem[];
-  float* s_in = smem;                                       // kSmStages windows (+ certainty windows)
-  float* s_y = smem + (CERT ? 2 : 1) * kSmStages * kSmWin;  // 2 y-result buffers
-  float* s_o = s_y + 2 * kSmYBuf;                           // 2 output planes
+  float* s_y = smem;                       // [8 planes][8 rows][kSmPY]
+  float* s_r = smem + kSmG * kSmYPlane;    // [2 groups][8 planes][8 rows][kSmPR]
   const int tid = threadIdx.x;
-  const int ntx = (W + kSmTX - 1) / kSmTX;
-  const int x0 = (int)(blockIdx.x % ntx) * kSmTX, y0 = (int)(blockIdx.x / ntx) * kSmTY;
+  const int ntx = (W + tw - 1) / tw;
+  const int x0 = (int)(blockIdx.x % ntx) * tw, y0 = (int)(blockIdx.x / ntx) * kSmTY;
   const int z0 = blockIdx.y * zc, z1 = min(D, z0 + zc);
-  const int np = z1 - z0 + 8;  // planes z0 - 4 .. z1 + 3
-  const long long WH = (long long)W * H;
-  const float* src = in + (long long)blockIdx.z * in_stride;
+  const int ngroups = (z1 - z0 + 8 + kSmG - 1) / kSmG;
+  const int WH = W * H;
+  const float* src = in + (long long)blockIdx.z * WH * D;
+  float* dst = out + (long long)blockIdx.z * WH * D;
 
-  // copies: window column wc (VEC wide), rows wr0 + RS m for m < NC
-  constexpr int CPR = kSmWX / VEC;            // copies per window row
-  constexpr int RS = kSmThreads / CPR;        // row step between a thread's copies
-  constexpr int NC = kSmWY / RS;              // copies per thread
-  static_assert(NC * RS == kSmWY, "window rows / thread mismatch");
-  const int wc = (tid % CPR) * VEC, wr0 = tid / CPR;
-  const int gx = x0 - 4 + wc;
-  const bool xin = gx >= 0 && gx < W;  // with VEC 2 and W even, gx + 1 < W too
-  unsigned rowmask = 0;
+  // y unit: plane yp of the group, window rows y0 - 4 .. y0 + 11, columns gx, gx + 1
+  const int ncp = (tw + 8) / 2;
+  const int yp = tid / ncp, yc = tid - yp * ncp;
+  const int gx = x0 - 4 + 2 * yc, gy = y0 - 4;
+  unsigned rows = 0;  // window rows inside the volume
 #pragma unroll
-  for (int m = 0; m < NC; m++) {
-    const int gy = y0 - 4 + wr0 + RS * m;
-    if (xin && gy >= 0 && gy < H) rowmask |= 1u << m;
-  }
-  // in-plane offset of copy 0 (outside the volume when its row is; only
-  // copies of rows inside the volume use it)
-  const long long off0 = (long long)(y0 - 4 + wr0) * W + gx;
-  const long long rstep = (long long)RS * W;
-  const uint32_t sdst0 = static_cast<uint32_t>(__cvta_generic_to_shared(s_in)) + 4u * (wr0 * kSmPitch + wc);
-  auto issue = [&](int k) {
-    const int p = z0 - 4 + k;
-    const bool pin = p >= 0 && p < D;
-    const unsigned mask = pin ? rowmask : 0u;
-    const long long poff = (long long)(pin ? p : 0) * WH;
-    const uint32_t d = sdst0 + 4u * (uint32_t)(((unsigned)k % kSmStages) * kSmWin);
+  for (int i = 0; i < 16; i++)
+    if (gy + i >= 0 && gy + i < H) rows |= 1u << i;
+  const bool in0 = gx >= 0 && gx < W, in1 = gx + 1 >= 0 && gx + 1 < W;
+  if ((!in0 && !in1) || yp >= kSmG) rows = 0;
+  const int yoff = gy * W + gx;  // in-plane offset of the first row (rows outside are not loaded)
+  float* const yb = s_y + yp * kSmYPlane + 2 * yc;
+  auto load = [&](const float* __restrict__ p, F2 (&a)[16]) {
+    const float* q = p + yoff;
+    if (VEC && rows == 0xffffu) {
 #pragma unroll
-    for (int m = 0; m < NC; m++) {
-      const bool v = (mask >> m) & 1u;
-      // copies outside the volume read nothing (size 0) from the volume's start
-      const long long o = v ? poff + off0 + m * rstep : 0;
-      cp_async<4 * VEC>(d + 4u * (uint32_t)(RS * m * kSmPitch), src + o, v ? 4u * VEC : 0u);
-      if (CERT) cp_async<4 * VEC>(d + 4u * (uint32_t)(kSmStages * kSmWin + RS * m * kSmPitch), cert + o,
-                                   v ? 4u * VEC : 0u);
-    }
-    cp_async_commit();
-  };
-  // y pass: window column yc, tile rows 4 yg .. 4 yg + 3
-  const int yc = tid & 63, yg = tid >> 6;
-  auto ypass = [&](int k) {
-    const float* w = s_in + ((unsigned)k % kSmStages) * kSmWin + (4 * yg) * kSmPitch + yc;
-    float* yb = s_y + (k & 1) * kSmYBuf + (4 * yg) * kSmPitch + yc;
-    float a[12];
+      for (int i = 0; i < 16; i++) a[i] = __ldg(reinterpret_cast<const F2*>(q + i * W));
+    } else {
 #pragma unroll
-    for (int i = 0; i < 12; i++) {
-      a[i] = w[i * kSmPitch];
-      if (CERT) a[i] *= w[kSmStages * kSmWin + i * kSmPitch];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      float sum = 0.f;
-#pragma unroll
-      for (int o = -4; o <= 4; o++) sum += a[i + 4 + o] * ty.f[4 - o];
-      yb[i * kSmPitch] = sum;
-    }
-  };
-  // x and z passes: tile row xr, outputs x0 + 4 xq .. + 3
-  const bool owner = tid < kSmOwners;
-  const int xr = tid / kSmXQ, xq = tid - (tid / kSmXQ) * kSmXQ;
-  float ring[9][4];
-#pragma unroll
-  for (int u = 0; u < 9; u++)
-#pragma unroll
-    for (int i = 0; i < 4; i++) ring[u][i] = 0.f;
-  // stores: tile row sr = tid / 16, columns sc + 16 i (i < 4, < 56)
-  const int sr = tid >> 4, sc = tid & 15;
-  unsigned colmask = 0;
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-    if (sc + 16 * i < kSmTX && x0 + sc + 16 * i < W) colmask |= 1u << i;
-  if (y0 + sr >= H) colmask = 0;
-  float* dst_row = out + (long long)blockIdx.z * out_stride + (long long)(y0 + sr) * W + x0 + sc;
-  const float* scert_row = DIV ? scert + (long long)(y0 + sr) * W + x0 + sc : nullptr;
-  auto store = [&](int j) {
-    const long long zoff = (long long)(z0 + j - 8) * WH;
-    const float* so = s_o + (j & 1) * kSmOut + sr * kSmTX + sc;
-    float* o = dst_row + zoff;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      if ((colmask >> i) & 1u) {
-        float q = so[16 * i];
-        if (DIV) q = q / __ldg(scert_row + zoff + 16 * i);
-        o[16 * i] = ACC ? o[16 * i] + q : q;
+      for (int i = 0; i < 16; i++) {
+        float2 v = make_float2(0.f, 0.f);
+        if ((rows >> i) & 1u) {
+          if (VEC) {
+            v = __ldg(reinterpret_cast<const float2*>(q + i * W));
+          } else {
+            if (in0) v.x = __ldg(q + i * W);
+            if (in1) v.y = __ldg(q + i * W + 1);
+          }
+        }
+        a[i] = f2_pack(v.x, v.y);
       }
+    }
+  };
+  // x units: row (lanes along the rows), plane and octet; at most two per thread
+  const int noct = tw / 8, nx = kSmG * kSmTY * noct;
+  int xp[2], xs[2], xd[2];
+#pragma unroll
+  for (int k = 0; k < 2; k++) {
+    const int u = tid + k * kSmThreads, row = u & 7, t = u >> 3;
+    const int pl = t / noct, oct = t - pl * noct;
+    xp[k] = u < nx ? pl : -1;
+    xs[k] = pl * kSmYPlane + row * kSmPY + 8 * oct;
+    xd[k] = pl * kSmRPlane + row * kSmPR + 8 * oct;
+  }
+  // z unit: one column pair of a row
+  const int ncz = tw / 2, zrow = tid / ncz, zcol = tid - zrow * ncz;
+  const int zx = x0 + 2 * zcol, zy = y0 + zrow;
+  const bool zon = zrow < kSmTY && zx < W && zy < H;
+  const bool two = VEC || zx + 1 < W;
+  const float* const zb = s_r + zrow * kSmPR + 2 * zcol;
+
+  // the group's z pass: chunk planes 8 (g - 1) .. 8 g + 7 sit in ring halves
+  // (g + 1) & 1 and g & 1; output plane i of the group sums planes i .. i + 8
+  // of those sixteen
+  auto zpass = [&](int g) {
+    if (!zon) return;
+    const int zo = z0 + kSmG * (g - 1);
+    F2 a[16];
+    const float* r0 = zb + ((g + 1) & 1) * kSmRGroup;
+    const float* r1 = zb + (g & 1) * kSmRGroup;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      a[i] = *reinterpret_cast<const F2*>(r0 + i * kSmRPlane);
+      a[8 + i] = *reinterpret_cast<const F2*>(r1 + i * kSmRPlane);
+    }
+    int o = zo * WH + zy * W + zx;
+#pragma unroll
+    for (int i = 0; i < kSmG; i++, o += WH) {
+      if (zo + i < z1) {
+        F2 sum = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) sum = f2_fma(a[i + j], taps.z[j], sum);
+        float2 v = f2_unpack(sum);
+        if (DIV) {
+          v.x = v.x / __ldg(scert + o);
+          if (two) v.y = v.y / __ldg(scert + o + 1);
+        }
+        if (MUL) {
+          v.x *= __ldg(cert + o);
+          if (two) v.y *= __ldg(cert + o + 1);
+        }
+        if (VEC) {
+          float2* d = reinterpret_cast<float2*>(dst + o);
+          if (ACC) {
+            const float2 old = *d;
+            v.x = old.x + v.x;
+            v.y = old.y + v.y;
+          }
+          *d = v;
+        } else {
+          dst[o] = ACC ? dst[o] + v.x : v.x;
+          if (two) dst[o + 1] = ACC ? dst[o + 1] + v.y : v.y;
+        }
+      }
+    }
   };
 
-  // planes 0 .. kSmStages - 2 in flight; plane 0 complete and visible
+  for (int g = 0; g <= ngroups; g++) {
+    // the z pass of the group before, then this group's loads and y pass
+    const int p = z0 - 4 + kSmG * g + yp;
+    const bool yin = g < ngroups && yp < kSmG && p >= 0 && p < D;
+    F2 a[16];
+    if (g >= 2) zpass(g - 1);
+    if (yin) {
+      load(src + (long long)p * WH, a);
+      if (CERT) {
+        F2 w[16];
+        load(cert + (long long)p * WH, w);
 #pragma unroll
-  for (int k = 0; k < kSmStages - 1; k++) {
-    if (k < np) issue(k);
-    else cp_async_commit();
-  }
-  cp_async_wait<kSmStages - 2>();
-  __syncthreads();
-  // phase k: copies of plane k + 3 issued, y pass of plane k, x and z passes
-  // of plane k - 1 (ring slot (k - 1) % 9), stores of plane k - 2; then plane
-  // k + 1 complete and visible
-  int slot = 0;
-  for (int k = 0; k <= np + 1; k++) {
-    if (k + kSmStages - 1 < np) issue(k + kSmStages - 1);
-    else cp_async_commit();
-    if (k < np) ypass(k);
-    if (k >= 1 && k <= np) {
-      if (owner) {
-        const int j = k - 1;
-        const float4* r4 = reinterpret_cast<const float4*>(s_y + (j & 1) * kSmYBuf + xr * kSmPitch + 4 * xq);
-        const float4 f0 = r4[0], f1 = r4[1], f2 = r4[2];
-        const float a[12] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w};
-        float v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          float sum = 0.f;
-#pragma unroll
-          for (int o = -4; o <= 4; o++) sum += a[i + 4 + o] * tx.f[4 - o];
-          v[i] = sum;
-        }
-        float4* od = reinterpret_cast<float4*>(s_o + (j & 1) * kSmOut + xr * kSmTX + 4 * xq);
-        // slot S holds plane j; the output plane z0 + j - 8 sums planes
-        // j - 8 .. j, held in slots S + 1 .. S + 9 (mod 9), oldest first
-#define BRC_SMOOTH_Z(S)                                                              \
-  case S: {                                                                          \
-    _Pragma("unroll") for (int i = 0; i < 4; i++) ring[S][i] = v[i];                 \
-    if (j >= 8) {                                                                    \
-      float zs[4];                                                                   \
-      _Pragma("unroll") for (int i = 0; i < 4; i++) {                                \
-        float sum = 0.f;                                                             \
-        _Pragma("unroll") for (int jj = 0; jj < 9; jj++) sum += ring[(S + 1 + jj) % 9][i] * tz.f[8 - jj]; \
-        zs[i] = sum;                                                                 \
-      }                                                                              \
-      *od = make_float4(zs[0], zs[1], zs[2], zs[3]);                                 \
-    }                                                                                \
-  } break;
-        switch (slot) {
-          BRC_SMOOTH_Z(0)
-          BRC_SMOOTH_Z(1)
-          BRC_SMOOTH_Z(2)
-          BRC_SMOOTH_Z(3)
-          BRC_SMOOTH_Z(4)
-          BRC_SMOOTH_Z(5)
-          BRC_SMOOTH_Z(6)
-          BRC_SMOOTH_Z(7)
-          BRC_SMOOTH_Z(8)
-        }
-#undef BRC_SMOOTH_Z
+        for (int i = 0; i < 16; i++) a[i] = f2_mul(a[i], w[i]);
       }
-      slot = slot == 8 ? 0 : slot + 1;
     }
-    if (k >= 10) store(k - 2);
-    cp_async_wait<kSmStages - 2>();
+    if (g == ngroups) break;
+    if (yin) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        F2 sum = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) sum = f2_fma(a[i + j], taps.y[j], sum);
+        *reinterpret_cast<F2*>(yb + i * kSmPY) = sum;
+      }
+    }
+    __syncthreads();
+    // x pass into ring half g & 1 (planes outside the volume: zeros)
+    float* const ring = s_r + (g & 1) * kSmRGroup;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+      if (xp[k] >= 0) {
+        const int zp = z0 - 4 + kSmG * g + xp[k];
+        F2 s[4] = {0, 0, 0, 0};
+        if (zp >= 0 && zp < D) {
+          const ulonglong2* r = reinterpret_cast<const ulonglong2*>(s_y + xs[k]);
+          F2 e[8], o[7];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            const ulonglong2 v = r[q];
+            e[2 * q] = v.x;
+            e[2 * q + 1] = v.y;
+          }
+#pragma unroll
+          for (int q = 0; q < 7; q++) o[q] = f2_pack(f2_unpack(e[q]).y, f2_unpack(e[q + 1]).x);
+#pragma unroll
+          for (int j = 0; j < 9; j++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) s[q] = f2_fma(j % 2 == 0 ? e[q + j / 2] : o[q + j / 2], taps.x[j], s[q]);
+        }
+        ulonglong2* d = reinterpret_cast<ulonglong2*>(ring + xd[k]);
+        d[0] = make_ulonglong2(s[0], s[1]);
+        d[1] = make_ulonglong2(s[2], s[3]);
+      }
+    }
     __syncthreads();
   }
-  cp_async_wait<0>();
 }
 
 // Planes per z chunk of smooth3d_kernel: enough chunks that the grid fills
@@ -1322,23 +1359,31 @@ cudaError_t multiply_mask(float* vols, const float* mask, long long V, int batch
 }
 
 // smooth3d_kernel instantiations indexed by (cert << 3) | (pairs << 2) |
-// (divide << 1) | accumulate.
+// (divide << 1) | accumulate, then the two of the normalised smoothing
+// (certainty, division, product with the certainty) by pairs.
 static const void* smooth_kernel_of(int v) {
-#define BRC_SK(C, P, Q, A) reinterpret_cast<const void*>(smooth3d_kernel<C, (P) ? 2 : 1, Q, A>)
-  static const void* const table[16] = {
-      BRC_SK(false, false, false, false), BRC_SK(false, false, false, true), BRC_SK(false, false, true, false),
-      BRC_SK(false, false, true, true),   BRC_SK(false, true, false, false), BRC_SK(false, true, false, true),
-      BRC_SK(false, true, true, false),   BRC_SK(false, true, true, true),   BRC_SK(true, false, false, false),
-      BRC_SK(true, false, false, true),   BRC_SK(true, false, true, false),  BRC_SK(true, false, true, true),
-      BRC_SK(true, true, false, false),   BRC_SK(true, true, false, true),   BRC_SK(true, true, true, false),
-      BRC_SK(true, true, true, true)};
+#define BRC_SK(C, P, Q, M, A) reinterpret_cast<const void*>(smooth3d_kernel<C, P, Q, M, A>)
+  static const void* const table[18] = {
+      BRC_SK(false, false, false, false, false), BRC_SK(false, false, false, false, true),
+      BRC_SK(false, false, true, false, false),  BRC_SK(false, false, true, false, true),
+      BRC_SK(false, true, false, false, false),  BRC_SK(false, true, false, false, true),
+      BRC_SK(false, true, true, false, false),   BRC_SK(false, true, true, false, true),
+      BRC_SK(true, false, false, false, false),  BRC_SK(true, false, false, false, true),
+      BRC_SK(true, false, true, false, false),   BRC_SK(true, false, true, false, true),
+      BRC_SK(true, true, false, false, false),   BRC_SK(true, true, false, false, true),
+      BRC_SK(true, true, true, false, false),    BRC_SK(true, true, true, false, true),
+      BRC_SK(true, false, true, true, false),    BRC_SK(true, true, true, true, false)};
 #undef BRC_SK
   return table[v];
 }
 
+static long long smooth_tiles(int W, int H) {
+  const int tw = smooth_tile_width(W);
+  return (long long)((W + tw - 1) / tw) * ((H + kSmTY - 1) / kSmTY);
+}
+
 int smooth3d_default_chunk(int W, int H, int D, int batch) {
-  const long long ntiles = (long long)((W + kSmTX - 1) / kSmTX) * ((H + kSmTY - 1) / kSmTY);
-  return smooth_chunk(D, ntiles * batch);
+  return smooth_chunk(D, smooth_tiles(W, H) * batch);
 }
 
 int smooth3d_chunk_candidates(int D, int* zc, int max_n) {
@@ -1355,14 +1400,16 @@ int smooth3d_chunk_candidates(int D, int* zc, int max_n) {
 
 cudaError_t smooth3d(const float* vol, int W, int H, int D, int batch, const float* fx,
                      const float* fy, const float* fz, const float* cert, const float* scert,
-                     float* tmp1, float* tmp2, float* out, cudaStream_t st, int accumulate, int zchunk) {
+                     float* tmp1, float* tmp2, float* out, cudaStream_t st, int accumulate, int zchunk,
+                     bool times_cert) {
   const long long V = (long long)W * H * D;
-  Taps9 tx, ty, tz;
+  SmoothTaps taps;
   for (int i = 0; i < 9; i++) {
-    tx.f[i] = fx[i];
-    ty.f[i] = fy[i];
-    tz.f[i] = fz[i];
+    taps.x[i] = f2_twice(fx[8 - i]);
+    taps.y[i] = f2_twice(fy[8 - i]);
+    taps.z[i] = f2_twice(fz[8 - i]);
   }
+  if (times_cert && (!cert || !scert || accumulate)) return cudaErrorInvalidValue;
   (void)tmp2;  // the fused kernel needs no second temporary
   // an output overlapping an input is computed into tmp1, then moved
   const size_t bytes = sizeof(float) * (size_t)V * batch;
@@ -1373,32 +1420,35 @@ cudaError_t smooth3d(const float* vol, int W, int H, int D, int batch, const flo
   const bool alias = overlaps(vol, bytes) || overlaps(cert, sizeof(float) * (size_t)V) ||
                      overlaps(scert, sizeof(float) * (size_t)V);
   float* dst = alias ? tmp1 : out;
-  const long long ntiles = (long long)((W + kSmTX - 1) / kSmTX) * ((H + kSmTY - 1) / kSmTY);
+  const long long ntiles = smooth_tiles(W, H);
   if (ntiles > 0x7fffffffLL || batch > 65535 || V > kMaxVoxels) return cudaErrorInvalidValue;
+  const int tw = smooth_tile_width(W);
   const int zc = zchunk > 0 ? (zchunk < D ? zchunk : D) : smooth_chunk(D, ntiles * batch);
   const dim3 grid((unsigned)ntiles, (unsigned)((D + zc - 1) / zc), (unsigned)batch);
   // the dynamic shared memory above 48 KB is a per-device function attribute
   static bool attr_set[64] = {false};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  // 8-byte copies need an even W (pairs never straddle the edge) and 8-byte
+  // 8-byte accesses need an even W (pairs never straddle the edge) and 8-byte
   // aligned volumes
-  const bool pairs = (W & 1) == 0 && ((reinterpret_cast<uintptr_t>(vol) | reinterpret_cast<uintptr_t>(cert)) & 7) == 0;
+  const bool pairs = (W & 1) == 0 &&
+                     ((reinterpret_cast<uintptr_t>(vol) | reinterpret_cast<uintptr_t>(cert) |
+                       reinterpret_cast<uintptr_t>(dst)) & 7) == 0;
   const bool acc = !alias && accumulate != 0;
-  const int variant = (cert ? 8 : 0) | (pairs ? 4 : 0) | (scert ? 2 : 0) | (acc ? 1 : 0);
+  const int variant = times_cert ? 16 + (pairs ? 1 : 0)
+                                 : (cert ? 8 : 0) | (pairs ? 4 : 0) | (scert ? 2 : 0) | (acc ? 1 : 0);
   if (!attr_set[dev]) {
-    for (int v = 0; v < 16; v++) {
-      const cudaError_t e0 = cudaFuncSetAttribute(smooth_kernel_of(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)smooth_smem_bytes((v & 8) != 0));
+    for (int v = 0; v < 18; v++) {
+      const cudaError_t e0 =
+          cudaFuncSetAttribute(smooth_kernel_of(v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmSmem);
       if (e0 != cudaSuccess) return e0;
     }
     attr_set[dev] = true;
   }
-  void* args[] = {(void*)&vol, (void*)&V, (void*)&cert, (void*)&scert, (void*)&W, (void*)&H, (void*)&D, (void*)&zc,
-                  (void*)&tx, (void*)&ty, (void*)&tz, (void*)&dst, (void*)&V};
+  void* args[] = {(void*)&vol, (void*)&cert, (void*)&scert, (void*)&W, (void*)&H,
+                  (void*)&D,   (void*)&tw,   (void*)&zc,    (void*)&taps, (void*)&dst};
   {
-    const cudaError_t e0 = cudaLaunchKernel(smooth_kernel_of(variant), grid, dim3(kSmThreads), args,
-                                            smooth_smem_bytes(cert != nullptr), st);
+    const cudaError_t e0 = cudaLaunchKernel(smooth_kernel_of(variant), grid, dim3(kSmThreads), args, kSmSmem, st);
     if (e0 != cudaSuccess) return e0;
   }
   cudaError_t e = cudaGetLastError();

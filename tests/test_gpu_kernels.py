@@ -162,3 +162,27 @@ def test_smooth_normalized_matches_golden(ctx):
     assert np.array_equal(np.isnan(out), np.isnan(ref))
     fin = np.isfinite(ref)
     assert np.abs(out[fin] - ref[fin]).max() <= TOL * np.abs(ref[fin]).max()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 8, 2), (9, 9, 63), (8, 7, 64), (17, 8, 65), (16, 17, 128), (33, 5, 130)])
+@pytest.mark.parametrize("weighted", [False, True])
+def test_smoothing_tile_edges_vs_oracle(ctx, orc, shape, weighted):
+    """Sizes at the edges of the smoothing's 64 x 8 tiles, octets and groups
+    of eight planes, with odd and even widths (single and paired accesses),
+    plain and as the normalised smoothing, whose quotient is multiplied by
+    the mask in the same kernel.  Same bar as the golden tests, 1e-4."""
+    rng = np.random.default_rng(sum(shape))
+    vols = rng.standard_normal((2,) + shape).astype(np.float32)
+    taps = [orc.smoothing_filter_sigma(s) for s in (1.0, 2.0, 5.0)]
+    if weighted:
+        mask = np.where(rng.random(shape) < 0.5, 1.0, 0.001).astype(np.float32)
+        sm = orc.smooth3d(mask, *taps)
+        got = ctx.smooth_normalized(cuda(vols), cuda(mask), *taps).cpu().numpy()
+        ref = [orc.smooth3d(v, *taps, mask, sm) * mask for v in vols]
+        parts = ctx.smooth3d(cuda(vols), *taps, cert=cuda(mask), smoothed_cert=ctx.smooth3d(cuda(mask), *taps))
+        assert np.array_equal(got, (parts * cuda(mask)).cpu().numpy())
+    else:
+        got = ctx.smooth3d(cuda(vols), *taps).cpu().numpy()
+        ref = [orc.smooth3d(v, *taps) for v in vols]
+    for b in range(2):
+        assert rel_err(got[b], ref[b]) < TOL
