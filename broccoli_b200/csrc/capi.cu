@@ -43,6 +43,15 @@ int pick_zpb(int W, int H) {
 
 }  // namespace
 
+// Volumes a filtering tuner times for launches of `batch`: the batch rounded
+// down to a power of two, at most 32 and at most 16 M voxels in all.
+static int timed_volumes(long long V, int batch) {
+  const long long most = (1ll << 24) / (V > 0 ? V : 1);
+  int nb = 1;
+  while (2 * nb <= batch && 2 * nb <= 32 && 2 * nb <= most) nb *= 2;
+  return nb;
+}
+
 static bool bad_dims(int W, int H, int D) {
   return W <= 0 || H <= 0 || D <= 0 || (long long)W * H * D > (1ll << 31);
 }
@@ -203,9 +212,11 @@ int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const floa
   return BRC_OK;
 }
 
-int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int* tz) {
+int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int batch, int* tz) {
   sym = sym && brc::filter3d_bank_symmetric(h_filters, nfilt);  // the kernel the launches will take
-  const auto key = std::make_tuple(nfilt + (sym ? 100 : 0), W, H, D);
+  const long long V = (long long)W * H * D;
+  const int nb = timed_volumes(V, batch);
+  const auto key = std::make_tuple(nfilt + (sym ? 100 : 0), W, H, D, nb);
   auto it = fp32_tuned.find(key);
   if (it != fp32_tuned.end()) {
     *tz = it->second;
@@ -220,9 +231,6 @@ int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H
   // time each z depth on zero-filled scratch volumes (the kernels' work does
   // not depend on the data, only on the shape and on whether the bank is
   // even/odd symmetric): one warm launch, best of three
-  const long long V = (long long)W * H * D;
-  long long nb = (1ll << 24) / (V > 0 ? V : 1);
-  nb = nb < 1 ? 1 : (nb > 32 ? 32 : nb);
   BRC_TRY(this, cudaStreamSynchronize(stream()), "synchronize");
   BRC_TRY(this, tmp1.ensure(sizeof(float) * (size_t)(V * nb)), "alloc");
   BRC_TRY(this, tmp2.ensure(sizeof(float) * (size_t)(V * nb) * 2 * nfilt), "alloc");
@@ -261,7 +269,7 @@ int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H
 }
 
 int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precision, int W, int H, int D,
-                     FilterPath* fp) {
+                     int batch, FilterPath* fp) {
   if (nfilt != 3 && nfilt != 6) return ctx->fail(BRC_ERR_INVALID, "filtering needs 3 or 6 filters");
   fp->precision = precision;
   fp->h_filters = h_filters;
@@ -269,7 +277,7 @@ int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precis
   fp->d_taps = nullptr;
   fp->d_err = ctx->tc_err.as<int>();
   if (precision == BRC_PREC_FP32 || precision == BRC_PREC_FP32_GENERAL)
-    return ctx->tune_fp32(h_filters, nfilt, precision == BRC_PREC_FP32, W, H, D, &fp->tz);
+    return ctx->tune_fp32(h_filters, nfilt, precision == BRC_PREC_FP32, W, H, D, batch, &fp->tz);
   if (precision != BRC_PREC_BF16X3 && precision != BRC_PREC_TF32)
     return ctx->fail(BRC_ERR_UNSUPPORTED, "unknown precision");
   const bool tf32 = precision == BRC_PREC_TF32;
@@ -429,7 +437,7 @@ int brc_filter3d(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batc
     return ctx->fail(BRC_ERR_INVALID, "brc_filter3d: vol_stride smaller than a volume");
   cudaSetDevice(ctx->device);
   FilterPath fp;
-  const int ps = make_filter_path(ctx, h_filters, nfilt, precision, W, H, D, &fp);
+  const int ps = make_filter_path(ctx, h_filters, nfilt, precision, W, H, D, batch, &fp);
   if (ps != BRC_OK) return ps;
   BRC_TRY(ctx, run_filter(fp, d_vol, W, H, D, batch, vol_stride, d_out, brc::all_instances(), ctx->stream()),
           "filter3d");
@@ -867,7 +875,7 @@ extern "C" int brc_register_linear_batched(brc_ctx* ctx, const float* d_ref, lon
   p.lists = p.status + 4;
   p.counts = p.lists + 3 * (size_t)batch;
   {
-    const int ps = make_filter_path(ctx, h_filters, 3, opts->precision, W, H, D, &p.fpath);
+    const int ps = make_filter_path(ctx, h_filters, 3, opts->precision, W, H, D, batch, &p.fpath);
     if (ps != BRC_OK) return ps;
   }
 

@@ -83,7 +83,8 @@ struct brc_ctx {
   DevBuf smask;   // smoothed certainty of brc_smooth_normalized
   // tensor-core tile height chosen by timing, per (nfilt, W, H, D)
   std::map<std::tuple<int, int, int, int>, int> tc_tuned;
-  std::map<std::tuple<int, int, int, int>, int> fp32_tuned;  // (nfilt + 100 sym, W, H, D) -> z depth
+  // (nfilt + 100 sym, W, H, D, volumes timed) -> z depth
+  std::map<std::tuple<int, int, int, int, int>, int> fp32_tuned;
   std::map<std::tuple<int, int, int, int, int>, int> smooth_tuned;  // (W, H, D, batch, cert kind) -> z chunk
   // host arrays of the debug outputs (brc_ctx_set_debug_outputs)
   bool dbg_on = false;
@@ -125,10 +126,12 @@ struct brc_ctx {
   // cost model's candidates, timed once per shape (outside stream capture;
   // under capture the cost model's first choice).
   int tune_tc(int nfilt, int W, int H, int D, const uint16_t* d_taps, bool tf32, int* ty);
-  // z depth of the FP32 filtering's output block for this shape and kind
-  // of kernel (even/odd when sym and the bank is symmetric, else general):
-  // the candidates timed once (outside stream capture), then cached.
-  int tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int* tz);
+  // z depth of the FP32 filtering's output block for this shape, launch size
+  // and kind of kernel (even/odd when sym and the bank is symmetric, else
+  // general): the candidates timed once (outside stream capture), then
+  // cached.  Launch sizes count by powers of two: a launch that does not fill
+  // the chip wants many small blocks, a large one few halos.
+  int tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int batch, int* tz);
   // brc::smooth3d with the z chunk tuned per (shape, batch, certainty
   // kind): the first call of a key that writes a buffer it does not read
   // and does not accumulate (outside stream capture) runs every candidate
@@ -161,8 +164,9 @@ struct FilterPath {
   int* d_err = nullptr;
   int tz = 0;  // FP32 filtering: z depth of the output block (0: untimed choice)
 };
+// batch: the volumes of the launches to come (any launch size is correct).
 int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precision, int W, int H, int D,
-                     FilterPath* fp);
+                     int batch, FilterPath* fp);
 inline bool brc_precision_valid(int p) {
   return p == BRC_PREC_FP32 || p == BRC_PREC_FP32_GENERAL || p == BRC_PREC_BF16X3 || p == BRC_PREC_TF32;
 }

@@ -85,6 +85,38 @@ __device__ __forceinline__ float sqrt_approx(float v) {
   return r;
 }
 
+// Two floats in one 64-bit register, and the packed operations on them; each
+// lane rounds as the scalar instruction does.
+typedef unsigned long long F2;
+__host__ __device__ __forceinline__ F2 f2_twice(float v) {
+  union {
+    float f[2];
+    F2 u;
+  } r;
+  r.f[0] = r.f[1] = v;
+  return r.u;
+}
+__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f2_unpack(F2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // OpenCL 1.2 section 8.2 linear filtering with unnormalised coordinates and
 // clamp-to-edge addressing, exact float weights (the sampler of
 // kernelRegistration.cpp:1064).  u, v, w include the +0.5 texel offset.

@@ -92,7 +92,7 @@ extern "C" int brc_tensor_magnitude(brc_ctx* ctx, const float* d_vol, int W, int
   BRC_TRY(ctx, q.ensure(sizeof(float) * 12 * V), "alloc");
   BRC_TRY(ctx, t.ensure(sizeof(float) * 6 * V + 64), "alloc");
   FilterPath fp;
-  FL_TRY(make_filter_path(ctx, h_filters6, 6, precision, W, H, D, &fp));
+  FL_TRY(make_filter_path(ctx, h_filters6, 6, precision, W, H, D, 1, &fp));
   BRC_TRY(ctx, run_filter(fp, d_vol, W, H, D, 1, V, q.as<float>(), brc::all_instances(), st), "filter");
   float* t6 = t.as<float>();
   BRC_TRY(ctx, brc::tensor_components(q.as<float>(), V, h_tensors, t6, st), "tensor_components");

@@ -923,38 +923,6 @@ constexpr int kSmRGroup = kSmG * kSmRPlane;
 constexpr size_t kSmSmem = sizeof(float) * (kSmG * kSmYPlane + 2 * kSmRGroup);
 static_assert(kSmTY == 8 && kSmG == 8, "the unit decodes assume 8 rows and groups of 8 planes");
 
-// Two floats in one 64-bit register, and the packed operations on them; each
-// lane rounds as the scalar instruction does.
-typedef unsigned long long F2;
-__host__ __device__ __forceinline__ F2 f2_twice(float v) {
-  union {
-    float f[2];
-    F2 u;
-  } r;
-  r.f[0] = r.f[1] = v;
-  return r.u;
-}
-__device__ __forceinline__ F2 f2_pack(float lo, float hi) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 f2_unpack(F2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
-  F2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
-  F2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 // The taps of the three passes, each twice (both lanes of a packed FMA), in
 // the order of the samples (o = -4..4 meets taps 8..0).
 struct SmoothTaps {
