@@ -219,8 +219,8 @@ normal_eq_partial_kernel(const float2* __restrict__ q1, long long q1_stride,
 //     shared-memory copy of the axis-1 responses of the adjacent warps (y)
 //     and from the previous / next plane held in registers (z);
 //   * each lane accumulates, over the planes, the FP32 moments
-//     sum w [1, z, z^2] and sum v [1, z] of its (x, y) column per axis and
-//     expands them once into the 42 FP64 sums with its x and y.
+//     sum w [1, z, z^2] and sum v [1, z] of its (x, y) column per axis, which
+//     are expanded once into the 42 FP64 sums.
 // The next plane's responses are loaded while the current plane's sums are
 // computed.  Without smoothing, the same sums as normal_eq_partial_kernel
 // up to FP32 summation order.
@@ -228,7 +228,11 @@ normal_eq_partial_kernel(const float2* __restrict__ q1, long long q1_stride,
 
 constexpr int kMarchWarps = 10;              // 8 output rows + 2 halo rows
 constexpr int kMarchCols = 30;               // output columns per warp
-constexpr int kMarchZs = 32;                 // at most this many planes per slab (16: 1 % slower)
+constexpr int kMarchZs = 32;                 // at most this many planes per slab (14: 3.5 % slower for a series)
+
+constexpr int kMarchRowSums = 27;            // 9 row moments per axis (below)
+// Row moment of sum e (0..13) of an axis: [s0, x s0, xx s0, sz, x sz, szz, v0, x v0, vz].
+__constant__ signed char c_row_moment[14] = {0, 1, 0, 3, 2, 1, 4, 0, 3, 5, 6, 7, 6, 8};
 
 struct PlaneQ {
   float2 a[3], c[3];  // q1, q2 of the three filters at this lane's (x, y)
@@ -258,7 +262,7 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
   __shared__ float cxr[SMOOTH ? 3 : 1][kMarchWarps][3][32];
   __shared__ float2 qy1[3][kMarchWarps][32];    // axis-1 responses (q1) of the last planes
   __shared__ float2 qy2[3][kMarchWarps][32];    // axis-1 responses (q2)
-  __shared__ double s_part[kMarchWarps][kNSums];
+  __shared__ double s_part[kMarchWarps][kMarchRowSums];
   const long long V = (long long)W * H * D;
   const long long WH = (long long)W * H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -350,10 +354,10 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
         for (int k = 0; k < 3; k++) {
           float pd, cert;
           phase_diff_cert(cur.a[k], cur.c[k], pd, cert);
+          const float g = phase_grad(ap[k], cur.a[k], am[k], cp[k], cur.c[k], cm[k]);
           if (SMOOTH)
             cert = w1 * cxr[SMOOTH ? j2 : 0][warp][k][lane] + w0 * cxr[SMOOTH ? j1 : 0][warp][k][lane] +
                    w1 * cxr[SMOOTH ? j : 0][warp][k][lane];  // planes z - 1, z, z + 1
-          const float g = phase_grad(ap[k], cur.a[k], am[k], cp[k], cur.c[k], cm[k]);
           const float cg = cert * g;
           const float wv = cg * g;
           const float vv = cg * pd;
@@ -379,40 +383,51 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
     }
   }
 
-  // expand the column moments into the 42 sums (FP64), warp sums, block sum
-  const double xd = (double)xf, yd = (double)y - 0.5 * (double)(H - 1);
+  // FP64 sums over the row of a warp (y is the same for its lanes): nine
+  // moments per axis, sum s0 [1, x, xx], sz [1, x], szz, v0 [1, x], vz.  The 27
+  // sums over 32 lanes take one transposing tree of 31 exchanges (lane l ends
+  // with sum l), not five shuffles per sum: the expansion of every lane into
+  // the 42 sums and their shuffles cost as much as two and a half planes
+  // (199 volumes of 64x64x33: 470 -> 437 us).
+  const double xd = (double)xf;
+  double red[32];
 #pragma unroll
-  for (int j = 0; j < kNSums; j++) {
-    const int k = j / 14, e = j % 14;
-    double v = 0.0;
-    if (out) {
-      const double s0 = m[k][0], sz = m[k][1], szz = m[k][2], v0 = m[k][3], vz = m[k][4];
-      switch (e) {
-        case 0: v = s0; break;
-        case 1: v = xd * s0; break;
-        case 2: v = yd * s0; break;
-        case 3: v = sz; break;
-        case 4: v = xd * xd * s0; break;
-        case 5: v = xd * yd * s0; break;
-        case 6: v = xd * sz; break;
-        case 7: v = yd * yd * s0; break;
-        case 8: v = yd * sz; break;
-        case 9: v = szz; break;
-        case 10: v = v0; break;
-        case 11: v = xd * v0; break;
-        case 12: v = yd * v0; break;
-        default: v = vz; break;
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) s_part[warp][j] = v;
+  for (int k = 0; k < 3; k++) {
+    const double s0 = m[k][0], sz = m[k][1], v0 = m[k][3];
+    red[9 * k] = s0;
+    red[9 * k + 1] = xd * s0;
+    red[9 * k + 2] = xd * xd * s0;
+    red[9 * k + 3] = sz;
+    red[9 * k + 4] = xd * sz;
+    red[9 * k + 5] = m[k][2];
+    red[9 * k + 6] = v0;
+    red[9 * k + 7] = xd * v0;
+    red[9 * k + 8] = m[k][4];
   }
+#pragma unroll
+  for (int i = kMarchRowSums; i < 32; i++) red[i] = 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool upper = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; i++) {
+      const double send = upper ? red[i] : red[i + o];
+      const double keep = upper ? red[i + o] : red[i];
+      red[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  if (lane < kMarchRowSums) s_part[warp][lane] = red[0];
   __syncthreads();
+  // the 42 sums from the eight output rows, in order
   if (threadIdx.x < kNSums) {
+    const int k = threadIdx.x / 14, e = threadIdx.x - 14 * k;
+    const int q = 9 * k + c_row_moment[e], py = c_sum_ypow[e];
     double v = 0.0;
 #pragma unroll
-    for (int w = 0; w < kMarchWarps; w++) v += s_part[w][threadIdx.x];
+    for (int w = 1; w <= 8; w++) {
+      const double yd = (double)(3 + yt * 8 - 1 + w) - 0.5 * (double)(H - 1);
+      v += s_part[w][q] * (py == 0 ? 1.0 : (py == 1 ? yd : yd * yd));
+    }
     partials[((long long)b * gridDim.x + blockIdx.x) * kNSums + threadIdx.x] = v;
   }
 }
@@ -426,11 +441,26 @@ __constant__ int c_mono_b[10] = {0, 0, 0, 0, 1, 1, 1, 2, 2, 3};
 
 __device__ __forceinline__ int axis_param(int k, int m) { return m == 0 ? k : 2 + 3 * k + m; }
 
-// Threads [0, 42) of the CTA sum the nblk partial rows of instance b.
+// Sums the nblk partial rows of instance b into s, in a fixed order: kRedSegs
+// threads per sum take every kRedSegs-th row, then the segments are added in
+// order.  (One thread per sum made this a chain of nblk dependent loads and
+// adds: 48 us at the 972 rows of a 182x218x182 volume.)
+constexpr int kRedSegs = 8;
+constexpr int kSolveThreads = 352;  // kRedSegs x 42 sums, whole warps
 __device__ void reduce_partials(const double* __restrict__ partials, int nblk, int b, double* s) {
+  __shared__ double seg_sum[kRedSegs][kNSums];
+  const int seg = threadIdx.x / kNSums, j = threadIdx.x - seg * kNSums;
+  if (seg < kRedSegs) {
+    double v = 0.0;
+#pragma unroll 4
+    for (int r = seg; r < nblk; r += kRedSegs) v += partials[((long long)b * nblk + r) * kNSums + j];
+    seg_sum[seg][j] = v;
+  }
+  __syncthreads();
   if (threadIdx.x < kNSums) {
     double v = 0.0;
-    for (int r = 0; r < nblk; r++) v += partials[((long long)b * nblk + r) * kNSums + threadIdx.x];
+#pragma unroll
+    for (int q = 0; q < kRedSegs; q++) v += seg_sum[q][threadIdx.x];
     s[threadIdx.x] = v;
   }
   __syncthreads();
@@ -456,92 +486,113 @@ __global__ void assemble_kernel(const double* __restrict__ partials, int nblk, d
   }
 }
 
-// Solves the 4x4 block of axis k by Gaussian elimination with complete
+// Solves the 4x4 block of an axis by Gaussian elimination with complete
 // pivoting.  Pivots at or below `thresh` end the elimination and the
 // remaining unknowns are 0, the rank rule of the reference's full-pivoting
-// QR solve (SolveEquationSystem, broccoli_lib.cpp:17157-17186).
-__device__ void solve4(double M[4][4], double r[4], double thresh, double x[4]) {
+// QR solve (SolveEquationSystem, broccoli_lib.cpp:17157-17186).  Every index
+// is a constant and the exchanges are selections, so that the matrix stays
+// in registers.
+__device__ __forceinline__ void swap_if(bool c, double& a, double& b) {
+  const double t = a;
+  a = c ? b : a;
+  b = c ? t : b;
+}
+__device__ __forceinline__ void solve4(double (&M)[4][4], double (&r)[4], double thresh, double (&x)[4]) {
   int perm[4] = {0, 1, 2, 3};
   int rank = 0;
+  bool on = true;
+#pragma unroll
   for (int k = 0; k < 4; k++) {
     int pr = k, pc = k;
     double best = -1.0;
+#pragma unroll
     for (int i = k; i < 4; i++)
-      for (int j = k; j < 4; j++)
-        if (fabs(M[i][j]) > best) {
-          best = fabs(M[i][j]);
-          pr = i;
-          pc = j;
-        }
-    if (best <= thresh || best == 0.0) break;
-    rank++;
-    if (pr != k) {
-      for (int j = 0; j < 4; j++) {
-        const double t = M[k][j];
-        M[k][j] = M[pr][j];
-        M[pr][j] = t;
+#pragma unroll
+      for (int j = k; j < 4; j++) {
+        const double m = fabs(M[i][j]);
+        const bool more = m > best;
+        best = more ? m : best;
+        pr = more ? i : pr;
+        pc = more ? j : pc;
       }
-      const double t = r[k];
-      r[k] = r[pr];
-      r[pr] = t;
+    on = on && !(best <= thresh || best == 0.0);
+    if (!on) continue;
+    rank = k + 1;
+#pragma unroll
+    for (int i = k + 1; i < 4; i++) {
+      const bool sw = pr == i;
+#pragma unroll
+      for (int j = 0; j < 4; j++) swap_if(sw, M[k][j], M[i][j]);
+      swap_if(sw, r[k], r[i]);
     }
-    if (pc != k) {
-      for (int i = 0; i < 4; i++) {
-        const double t = M[i][k];
-        M[i][k] = M[i][pc];
-        M[i][pc] = t;
-      }
+#pragma unroll
+    for (int j = k + 1; j < 4; j++) {
+      const bool sw = pc == j;
+#pragma unroll
+      for (int i = 0; i < 4; i++) swap_if(sw, M[i][k], M[i][j]);
       const int t = perm[k];
-      perm[k] = perm[pc];
-      perm[pc] = t;
+      perm[k] = sw ? perm[j] : perm[k];
+      perm[j] = sw ? t : perm[j];
     }
+#pragma unroll
     for (int i = k + 1; i < 4; i++) {
       const double m = M[i][k] / M[k][k];
-      if (m == 0.0) continue;
-      for (int j = k; j < 4; j++) M[i][j] -= m * M[k][j];
-      r[i] -= m * r[k];
+      if (m != 0.0) {
+#pragma unroll
+        for (int j = k; j < 4; j++) M[i][j] -= m * M[k][j];
+        r[i] -= m * r[k];
+      }
     }
   }
   double y[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = rank - 1; i >= 0; i--) {
-    double s = r[i];
-    for (int j = i + 1; j < rank; j++) s -= M[i][j] * y[j];
-    y[i] = s / M[i][i];
+#pragma unroll
+  for (int i = 3; i >= 0; i--) {
+    if (i < rank) {
+      double s = r[i];
+#pragma unroll
+      for (int j = i + 1; j < 4; j++)
+        if (j < rank) s -= M[i][j] * y[j];
+      y[i] = s / M[i][i];
+    }
   }
-  for (int i = 0; i < 4; i++) x[perm[i]] = y[i];
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    double v = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) v = perm[i] == q ? y[i] : v;
+    x[q] = v;
+  }
 }
 
-// p = A^-1 h for the 12-parameter system given by the 42 sums, FP64,
-// rounded to float (the reference casts its Eigen solution to float).
-__device__ void solve12_from_sums(const double* s, float p[12]) {
+// The four parameters of axis k from the 42 sums, FP64, rounded to float (the
+// reference casts its Eigen solution to float): one thread per axis.
+__device__ __forceinline__ void solve_axis_from_sums(const double* s, int k, float* p) {
   double maxabs = 0.0;
   for (int j = 0; j < kNSums; j++)
     if ((j % 14) < 10) maxabs = fmax(maxabs, fabs(s[j]));
   const double thresh = maxabs * 2.220446049250313e-16 * 12.0;
-  for (int k = 0; k < 3; k++) {
-    double M[4][4], r[4], x[4];
-    for (int e = 0; e < 10; e++) {
-      const int a = c_mono_a[e], bb = c_mono_b[e];
-      M[a][bb] = s[14 * k + e];
-      M[bb][a] = s[14 * k + e];
-    }
-    for (int m = 0; m < 4; m++) r[m] = s[14 * k + 10 + m];
-    solve4(M, r, thresh, x);
-    for (int m = 0; m < 4; m++) p[axis_param(k, m)] = (float)x[m];
-  }
+  const double* e = s + 14 * k;
+  double M[4][4] = {{e[0], e[1], e[2], e[3]}, {e[1], e[4], e[5], e[6]}, {e[2], e[5], e[7], e[8]}, {e[3], e[6], e[8], e[9]}};
+  double r[4] = {e[10], e[11], e[12], e[13]}, x[4];
+  solve4(M, r, thresh, x);
+#pragma unroll
+  for (int m = 0; m < 4; m++) p[axis_param(k, m)] = (float)x[m];
 }
 
 // Orthogonal polar factor U V^T of a 3x3 matrix (row-major) from one-sided
 // Jacobi sweeps, FP64 (the reference takes U V^T of Eigen's JacobiSVD in
 // RemoveTransformationScaling, broccoli_lib.cpp:6153-6194).
-__device__ void polar3(const double* M, double* R) {
+__device__ __forceinline__ void polar3(const double* M, double* R) {
   double A[9], Vm[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1};
   for (int i = 0; i < 9; i++) A[i] = M[i];
   for (int sweep = 0; sweep < 60; sweep++) {
     bool rotated = false;
+#pragma unroll
     for (int p = 0; p < 2; p++)
+#pragma unroll
       for (int q = p + 1; q < 3; q++) {
         double al = 0, be = 0, ga = 0;
+#pragma unroll
         for (int i = 0; i < 3; i++) {
           al += A[i * 3 + p] * A[i * 3 + p];
           be += A[i * 3 + q] * A[i * 3 + q];
@@ -552,6 +603,7 @@ __device__ void polar3(const double* M, double* R) {
         const double zeta = (be - al) / (2.0 * ga);
         const double t = (zeta >= 0 ? 1.0 : -1.0) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
         const double c = 1.0 / sqrt(1.0 + t * t), sn = c * t;
+#pragma unroll
         for (int i = 0; i < 3; i++) {
           const double ap = A[i * 3 + p], aq = A[i * 3 + q];
           A[i * 3 + p] = c * ap - sn * aq;
@@ -564,10 +616,12 @@ __device__ void polar3(const double* M, double* R) {
     if (!rotated) break;
   }
   double U[9], sig[3];
+#pragma unroll
   for (int j = 0; j < 3; j++) {
     sig[j] = sqrt(A[j] * A[j] + A[3 + j] * A[3 + j] + A[6 + j] * A[6 + j]);
     for (int i = 0; i < 3; i++) U[i * 3 + j] = sig[j] > 0 ? A[i * 3 + j] / sig[j] : 0.0;
   }
+#pragma unroll
   for (int j = 0; j < 3; j++)
     if (!(sig[j] > 0)) {
       const int a = (j + 1) % 3, bb = (j + 2) % 3;
@@ -575,7 +629,9 @@ __device__ void polar3(const double* M, double* R) {
       U[1 * 3 + j] = U[2 * 3 + a] * U[0 * 3 + bb] - U[0 * 3 + a] * U[2 * 3 + bb];
       U[2 * 3 + j] = U[0 * 3 + a] * U[1 * 3 + bb] - U[1 * 3 + a] * U[0 * 3 + bb];
     }
+#pragma unroll
   for (int i = 0; i < 3; i++)
+#pragma unroll
     for (int j = 0; j < 3; j++) {
       double s = 0;
       for (int k = 0; k < 3; k++) s += U[i * 3 + k] * Vm[j * 3 + k];
@@ -648,14 +704,15 @@ __device__ void rotation_angles(const float* p, float* rot) {
 __device__ double update_magnitude(const float* p, int W, int H, int D) {
   const double hx = 0.5 * (W - 1), hy = 0.5 * (H - 1), hz = 0.5 * (D - 1);
   double best = 0.0;
+#pragma unroll
   for (int c = 0; c < 8; c++) {
     const double x = (c & 1) ? hx : -hx, y = (c & 2) ? hy : -hy, z = (c & 4) ? hz : -hz;
     const double dx = p[0] + p[3] * x + p[4] * y + p[5] * z;
     const double dy = p[1] + p[6] * x + p[7] * y + p[8] * z;
     const double dz = p[2] + p[9] * x + p[10] * y + p[11] * z;
-    best = fmax(best, sqrt(dx * dx + dy * dy + dz * dz));
+    best = fmax(best, dx * dx + dy * dy + dz * dz);
   }
-  return best;
+  return sqrt(best);
 }
 
 // One iteration's solve and parameter update for every active instance
@@ -675,10 +732,15 @@ __global__ void solve_update_kernel(const double* __restrict__ partials, int nbl
   if (blockIdx.x == 0 && threadIdx.x == 0) counts[(it + 2) % 3] = 0;
   if ((int)blockIdx.x >= active_count(act, (int)gridDim.x)) return;
   const int b = active_instance(act, blockIdx.x);
+  __shared__ float s_p[12];
   reduce_partials(partials, nblk, b, s);
+  // three warps, one axis each; then thread 0
+  if ((threadIdx.x & 31) == 0 && threadIdx.x < 96) solve_axis_from_sums(s, threadIdx.x >> 5, s_p);
+  __syncthreads();
   if (threadIdx.x != 0) return;
   float p[12];
-  solve12_from_sums(s, p);
+#pragma unroll
+  for (int i = 0; i < 12; i++) p[i] = s_p[i];
   bool finite = true;
   for (int i = 0; i < 12; i++) finite = finite && isfinite(p[i]);
   if (!finite) {
@@ -1171,7 +1233,7 @@ cudaError_t normal_eq_march(const float* q1, long long q1_stride_floats, const f
 
 cudaError_t assemble_normal_eq(const double* partials, int nblk, int batch, double* A, double* h,
                                cudaStream_t st) {
-  assemble_kernel<<<batch, 64, 0, st>>>(partials, nblk, A, h);
+  assemble_kernel<<<batch, kSolveThreads, 0, st>>>(partials, nblk, A, h);
   return cudaGetLastError();
 }
 
@@ -1179,7 +1241,7 @@ cudaError_t solve_update(const double* partials, int nblk, int batch, int type, 
                          int H, int D, float* params, float* rotations, int* conv_iter,
                          int* iterations, int* status, ActiveSet act, int* lists, int* counts, cudaStream_t st) {
   if (!act.list) return cudaErrorInvalidValue;
-  solve_update_kernel<<<batch, 64, 0, st>>>(partials, nblk, type, tol, W, H, D, params, rotations,
+  solve_update_kernel<<<batch, kSolveThreads, 0, st>>>(partials, nblk, type, tol, W, H, D, params, rotations,
                                             conv_iter, iterations, status, act, lists, counts);
   return cudaGetLastError();
 }
