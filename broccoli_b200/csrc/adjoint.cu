@@ -16,79 +16,166 @@
 
 namespace brc {
 
-constexpr int kAdjTX = 32, kAdjTY = 8, kAdjTZ = 4, kAdjR = 8, kAdjRowPad = 44;
-constexpr int kAdjThreads = (kAdjTX / kAdjR) * kAdjTY * kAdjTZ;  // 128
+// One CTA computes a 32 x 16 x 4 block of outputs; a thread owns 4 (x) x 4
+// (y) of them.  The gradient of one filter at a time is staged in shared
+// memory as (re, im) pairs with its +-3 halo, and each pair meets the tap
+// pair (W_re, W_im) in one packed FMA whose lanes accumulate the real and
+// the imaginary channel's part of the sum, added at the end.
+//
+// Every staged sample feeds one real output per tap only, so shared-memory
+// bandwidth, not the FMA pipe, bounds the plain form (a row segment per
+// (dz, dy): 16 samples loaded for 56 FMAs, and the two channels of a filter
+// staged one after the other with stride-2 reads).  Four output rows per
+// thread reuse a loaded row for up to four dy: 6 + 16 shared loads (40
+// wavefronts) per 112 packed FMAs (224 cycles of a scheduler's FMA pipe).
+// The rows yr = 0..9 of a thread's window meet output y with dy = yr - y in
+// 0..6; the rows 3..6 meet all four outputs and run as a loop, the three
+// before and after are unrolled (one body for all ten would be half zeros,
+// ten bodies would not fit the instruction cache).
+//
+// Bank conflicts: a quarter-warp's 16-byte loads come from four x groups (2
+// slots of 16 bytes apart) of two slices, whose pitch is odd in slots.
+//
+// The copies of a filter's block (70 KB) are all in flight at once (cp.async);
+// loading it through registers, four at a time, took a third of the kernel.
+// Three filters at 128x128x96: 276 us (one row segment per (dz, dy)) -> 228
+// (four rows per thread) -> 170 (cp.async).  At this size the grid is 1.7
+// waves of three blocks per SM.
+constexpr int kAdjTX = 32, kAdjTY = 16, kAdjTZ = 4;
+constexpr int kAdjR = 4, kAdjY = 4;
+constexpr int kAdjThreads = (kAdjTX / kAdjR) * (kAdjTY / kAdjY) * kAdjTZ;  // 128
+constexpr int kAdjRow = kAdjTX + 8;                                        // pairs of a staged row (38 used)
+constexpr int kAdjRows = kAdjTY + 6, kAdjSlices = kAdjTZ + 6;
+constexpr int kAdjSlice = kAdjRows * kAdjRow + 2;  // pairs: 441 slots of 16 bytes
+constexpr int kAdjWRow = 8;                        // tap pairs of a (dz, dy) row (7 used)
+constexpr size_t kAdjSmem = 8 * ((size_t)kAdjSlices * kAdjSlice + 49 * kAdjWRow);
+static_assert((kAdjSlice / 2) % 2 == 1 && kAdjThreads == 128, "bank layout / thread decode");
 
 template <int NF>
 struct AdjBank {
-  float w[2 * NF][kTaps];  // channel c = 2k + (0 re, 1 im); index (ex+3) + 7(ey+3) + 49(ez+3)
+  float2 w[NF][kTaps];  // (re, im) of filter k; index (ex+3) + 7(ey+3) + 49(ez+3)
 };
 
 template <int NF>
-__global__ void __launch_bounds__(kAdjThreads)
+__global__ void __launch_bounds__(kAdjThreads, 3)
 filter3d_adjoint_kernel(const float* __restrict__ grad, int W, int H, int D,
                         const __grid_constant__ AdjBank<NF> bank, float* __restrict__ out) {
-  constexpr int kRows = kAdjTY + 6, kSlices = kAdjTZ + 6;
-  __shared__ __align__(16) float s_vol[kSlices * kRows * kAdjRowPad];
-  __shared__ __align__(16) float s_w[kTaps];
+  extern __shared__ __align__(16) F2 adj_smem[];
+  F2* s_g = adj_smem;
+  F2* s_w = adj_smem + kAdjSlices * kAdjSlice;
   const int b = blockIdx.z;
   const int z_tiles = (D + kAdjTZ - 1) / kAdjTZ;
   const int tile_x0 = blockIdx.x * kAdjTX;
   const int tile_y0 = (blockIdx.y / z_tiles) * kAdjTY;
   const int tile_z0 = (blockIdx.y % z_tiles) * kAdjTZ;
   const long long V = (long long)W * H * D;
-  const int tx = threadIdx.x % (kAdjTX / kAdjR);
-  const int ty = (threadIdx.x / (kAdjTX / kAdjR)) % kAdjTY;
-  const int tz = threadIdx.x / ((kAdjTX / kAdjR) * kAdjTY);
-  float acc[kAdjR];
+  // lanes: x group (low two bits), slice (low bit), x group (high bit), slice (high bit)
+  const int lane = threadIdx.x & 31, yg = threadIdx.x >> 5;
+  const int tx = (lane & 3) | ((lane >> 1) & 4), tz = ((lane >> 2) & 1) | ((lane >> 3) & 2);
+  const int xl = threadIdx.x & 7;
+  // pairs move as 8 bytes where the gradient is 8-byte aligned
+  const bool pairs = (reinterpret_cast<uintptr_t>(grad) & 7) == 0;
+
+  F2 acc[kAdjY][kAdjR];
 #pragma unroll
-  for (int r = 0; r < kAdjR; r++) acc[r] = 0.f;
+  for (int y = 0; y < kAdjY; y++)
+#pragma unroll
+    for (int r = 0; r < kAdjR; r++) acc[y][r] = 0;
 
 #pragma unroll 1
-  for (int c = 0; c < 2 * NF; c++) {
-    const float* g = grad + ((long long)b * NF + (c >> 1)) * 2 * V + (c & 1);
+  for (int k = 0; k < NF; k++) {
+    const float* g = grad + ((long long)b * NF + k) * 2 * V;
     __syncthreads();
-    for (int i = threadIdx.x; i < kTaps; i += kAdjThreads) s_w[i] = bank.w[c][i];
-    for (int i = threadIdx.x; i < kSlices * kRows * kAdjRowPad; i += kAdjThreads) {
-      const int xs = i % kAdjRowPad, ys = (i / kAdjRowPad) % kRows, zs = i / (kAdjRowPad * kRows);
-      const int x = tile_x0 - 4 + xs, y = tile_y0 - 3 + ys, z = tile_z0 - 3 + zs;
-      float v = 0.f;
-      if (x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D)
-        v = __ldg(g + 2 * (x + (long long)y * W + (long long)z * W * H));
-      s_vol[i] = v;
+    for (int i = threadIdx.x; i < 49 * kAdjWRow; i += kAdjThreads) {
+      const int row = i / kAdjWRow, dx = i % kAdjWRow;
+      const float2 w = dx < 7 ? bank.w[k][row * 7 + dx] : make_float2(0.f, 0.f);
+      s_w[i] = f2_pack(w.x, w.y);
     }
-    __syncthreads();
-#pragma unroll 1
-    for (int dz = 0; dz < 7; dz++) {
-#pragma unroll 1
-      for (int dy = 0; dy < 7; dy++) {
-        const float4* row = reinterpret_cast<const float4*>(
-            s_vol + ((tz + dz) * kRows + (ty + dy)) * kAdjRowPad + kAdjR * tx);
-        float d[16];
+    // eight threads copy a row, every copy in flight at once
+    for (int row = threadIdx.x >> 3; row < kAdjSlices * kAdjRows; row += kAdjThreads / 8) {
+      const int zs = row / kAdjRows, ys = row - zs * kAdjRows;
+      const int y = tile_y0 - 3 + ys, z = tile_z0 - 3 + zs;
+      const bool rowok = y >= 0 && y < H && z >= 0 && z < D;
+      const float* q = g + 2 * ((long long)(rowok ? y : 0) * W + (long long)(rowok ? z : 0) * W * H);
+      const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(s_g + zs * kAdjSlice + ys * kAdjRow)) + 8 * xl;
 #pragma unroll
-        for (int s = 0; s < 4; s++) {
-          const float4 q = row[s];
-          d[4 * s] = q.x;
-          d[4 * s + 1] = q.y;
-          d[4 * s + 2] = q.z;
-          d[4 * s + 3] = q.w;
-        }
-        const float* wr = s_w + dy * 7 + dz * 49;
-#pragma unroll
-        for (int dx = 0; dx < 7; dx++) {
-          const float w = wr[dx];
-#pragma unroll
-          for (int r = 0; r < kAdjR; r++) acc[r] = fmaf(d[1 + r + dx], w, acc[r]);
+      for (int m = 0; m < kAdjRow / 8; m++) {
+        const int x = tile_x0 - 4 + xl + 8 * m;
+        const bool ok = rowok && x >= 0 && x < W;
+        const float* p = q + (ok ? 2 * x : 0);
+        if (pairs) {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d + 64 * m), "l"(p), "r"(ok ? 8 : 0) : "memory");
+        } else {
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 64 * m), "l"(p), "r"(ok ? 4 : 0) : "memory");
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 64 * m + 4), "l"(p + 1), "r"(ok ? 4 : 0)
+                       : "memory");
         }
       }
     }
-  }
-  const int x0 = tile_x0 + kAdjR * tx, y = tile_y0 + ty, z = tile_z0 + tz;
-  if (y >= H || z >= D) return;
-  float* o = out + (long long)b * V + x0 + (long long)y * W + (long long)z * W * H;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+#pragma unroll 1
+    for (int dz = 0; dz < 7; dz++) {
+      const F2* rows = s_g + (tz + dz) * kAdjSlice + (kAdjY * yg) * kAdjRow + kAdjR * tx;
+      const F2* taps = s_w + dz * 7 * kAdjWRow;
+      F2 d[12];
+      // sample at offset ex of output r sits at d[4 + r + ex]
+      auto load_row = [&](int yr) {
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(rows + yr * kAdjRow);
 #pragma unroll
-  for (int r = 0; r < kAdjR; r++)
-    if (x0 + r < W) o[r] = acc[r];
+        for (int s = 0; s < 6; s++) {
+          const ulonglong2 v = q[s];
+          d[2 * s] = v.x;
+          d[2 * s + 1] = v.y;
+        }
+      };
+      auto add = [&](F2 (&o)[kAdjR], int dy) {
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(taps + dy * kAdjWRow);
+#pragma unroll
+        for (int s = 0; s < 4; s++) {
+          const ulonglong2 w = q[s];
+#pragma unroll
+          for (int r = 0; r < kAdjR; r++) o[r] = f2_fma(d[1 + r + 2 * s], w.x, o[r]);
+          if (s < 3) {
+#pragma unroll
+            for (int r = 0; r < kAdjR; r++) o[r] = f2_fma(d[2 + r + 2 * s], w.y, o[r]);
+          }
+        }
+      };
+#pragma unroll
+      for (int yr = 0; yr < 3; yr++) {
+        load_row(yr);
+#pragma unroll
+        for (int y = 0; y <= yr; y++) add(acc[y], yr - y);
+      }
+#pragma unroll 1
+      for (int yr = 3; yr < 7; yr++) {
+        load_row(yr);
+#pragma unroll
+        for (int y = 0; y < kAdjY; y++) add(acc[y], yr - y);
+      }
+#pragma unroll
+      for (int yr = 7; yr < 10; yr++) {
+        load_row(yr);
+#pragma unroll
+        for (int y = yr - 6; y < kAdjY; y++) add(acc[y], yr - y);
+      }
+    }
+  }
+  const int x0 = tile_x0 + kAdjR * tx, z = tile_z0 + tz;
+  if (z >= D) return;
+#pragma unroll
+  for (int yy = 0; yy < kAdjY; yy++) {
+    const int y = tile_y0 + kAdjY * yg + yy;
+    if (y >= H) break;
+    float* o = out + (long long)b * V + x0 + (long long)y * W + (long long)z * W * H;
+#pragma unroll
+    for (int r = 0; r < kAdjR; r++)
+      if (x0 + r < W) {
+        const float2 v = f2_unpack(acc[yy][r]);
+        o[r] = v.x + v.y;
+      }
+  }
 }
 
 // Value and gradient (d/du, d/dv, d/dw) of the clamp-to-edge trilinear
@@ -195,12 +282,15 @@ warp_affine_backward_kernel(const float* __restrict__ src, int W, int H, int D,
   }
 }
 
+// out[b][j] = sum of the nblk partial rows, one warp per sum: lane l takes
+// rows l, l + 32, .., then a fixed shuffle tree (the same order on every run).
 __global__ void reduce12_kernel(const double* __restrict__ partials, int nblk, double* __restrict__ out) {
-  const int b = blockIdx.x, j = threadIdx.x;
-  if (j >= 12) return;
+  const int b = blockIdx.x, j = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double v = 0.0;
-  for (int r = 0; r < nblk; r++) v += partials[((long long)b * nblk + r) * 12 + j];
-  out[(long long)b * 12 + j] = v;
+  for (int r = lane; r < nblk; r += 32) v += partials[((long long)b * nblk + r) * 12 + j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (lane == 0) out[(long long)b * 12 + j] = v;
 }
 
 // Field warp backward: dL/du per voxel and optionally dL/dsrc.
@@ -236,16 +326,26 @@ static cudaError_t launch_adjoint(const float* grad, int W, int H, int D, int ba
                                   float* out, cudaStream_t st) {
   AdjBank<NF> bank;
   for (int k = 0; k < NF; k++)
-    for (int c = 0; c < 2; c++)
-      for (int ez = -3; ez <= 3; ez++)
-        for (int ey = -3; ey <= 3; ey++)
-          for (int ex = -3; ex <= 3; ex++)
-            // weight W(-e) = F[3 + e]
-            bank.w[2 * k + c][(ex + 3) + 7 * (ey + 3) + 49 * (ez + 3)] =
-                h_filters[k * kFilterFloats + c * kTaps + (3 + ex) + 7 * (3 + ey) + 49 * (3 + ez)];
+    for (int ez = -3; ez <= 3; ez++)
+      for (int ey = -3; ey <= 3; ey++)
+        for (int ex = -3; ex <= 3; ex++) {
+          // weight W(-e) = F[3 + e]
+          const float* f = h_filters + k * kFilterFloats + (3 + ex) + 7 * (3 + ey) + 49 * (3 + ez);
+          bank.w[k][(ex + 3) + 7 * (ey + 3) + 49 * (ez + 3)] = make_float2(f[0], f[kTaps]);
+        }
+  // the dynamic shared memory above 48 KB is a per-device function attribute
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (!attr_set[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(filter3d_adjoint_kernel<NF>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAdjSmem);
+    if (e != cudaSuccess) return e;
+    attr_set[dev] = true;
+  }
   const int z_tiles = (D + kAdjTZ - 1) / kAdjTZ;
   dim3 grid((W + kAdjTX - 1) / kAdjTX, ((H + kAdjTY - 1) / kAdjTY) * z_tiles, batch);
-  filter3d_adjoint_kernel<NF><<<grid, kAdjThreads, 0, st>>>(grad, W, H, D, bank, out);
+  filter3d_adjoint_kernel<NF><<<grid, kAdjThreads, kAdjSmem, st>>>(grad, W, H, D, bank, out);
   return cudaGetLastError();
 }
 
@@ -266,7 +366,7 @@ cudaError_t warp_affine_backward(const float* src, int W, int H, int D, int batc
                                  cudaStream_t st) {
   dim3 grid(nblk, batch);
   warp_affine_backward_kernel<<<grid, kWBThreads, 0, st>>>(src, W, H, D, params, gout, partials, gsrc);
-  reduce12_kernel<<<batch, 32, 0, st>>>(partials, nblk, gparams);
+  reduce12_kernel<<<batch, 12 * 32, 0, st>>>(partials, nblk, gparams);
   return cudaGetLastError();
 }
 

@@ -171,3 +171,31 @@ def test_gradients_at_full_config_size(orc, lin_filters):
         gg.append(gf[c, z, y, x])
     fdf, gg = np.array(fdf), np.array(gg)
     assert np.abs(gg - fdf).max() <= 1e-3 * np.abs(fdf).max(), (gg, fdf)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (4, 16, 32), (5, 17, 33), (3, 31, 65), (9, 15, 31)])
+@pytest.mark.parametrize("nf", [3, 6])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_filter_adjoint_tile_edges(shape, nf, offset, bank):
+    """brc_filter3d_adjoint at the edges of its 32 x 16 x 4 blocks, two
+    volumes, with a gradient that is 8-byte aligned and one that is not,
+    against the transpose of the convolution in FP64 (torch on the CPU): the
+    adjoint is the cross-correlation with the unflipped filters.  FP32 bar of
+    the suite, 1e-4 of the largest value."""
+    flt = bank["linear" if nf == 3 else "nonlinear"]
+    D, H, W = shape
+    gen = torch.Generator().manual_seed(sum(shape) + nf)
+    g = torch.randn((2, nf) + shape + (2,), generator=gen)
+    ref = torch.nn.functional.conv3d(
+        torch.movedim(g.double(), -1, 2).reshape(2, 2 * nf, D, H, W),
+        torch.from_numpy(flt).double().reshape(1, 2 * nf, 7, 7, 7), padding=3)[:, 0]
+    buf = torch.empty(g.numel() + 1, device="cuda")
+    gd = buf[offset:offset + g.numel()]
+    gd.copy_(g.reshape(-1))
+    out = torch.full((2,) + shape, float("nan"), device="cuda")
+    c = AG._ctx(out.device)
+    fn = AG._sig("brc_filter3d_adjoint", [AG._P, AG._P, AG._I, AG._I, AG._I, AG._I, AG._P, AG._I, AG._P])
+    f = np.ascontiguousarray(flt, np.float32)
+    assert fn(c.handle, AG._p(gd), W, H, D, 2, f.ctypes.data, nf, AG._p(out)) == 0
+    err = (out.cpu().double() - ref).abs().max() / ref.abs().max()
+    assert float(err) < 1e-4
