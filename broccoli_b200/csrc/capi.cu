@@ -212,11 +212,10 @@ int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const floa
   return BRC_OK;
 }
 
-int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int batch, int* tz) {
-  sym = sym && brc::filter3d_bank_symmetric(h_filters, nfilt);  // the kernel the launches will take
+int brc_ctx::tune_fp32(const float* bank, brc::FilterKind kind, int nfilt, int W, int H, int D, int batch, int* tz) {
   const long long V = (long long)W * H * D;
   const int nb = timed_volumes(V, batch);
-  const auto key = std::make_tuple(nfilt + (sym ? 100 : 0), W, H, D, nb);
+  const auto key = std::make_tuple(nfilt + (kind == brc::kFilterSym ? 100 : 0), W, H, D, nb);
   auto it = fp32_tuned.find(key);
   if (it != fp32_tuned.end()) {
     *tz = it->second;
@@ -248,8 +247,8 @@ int brc_ctx::tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H
     for (int rep = 0; rep < 4 && err == cudaSuccess; rep++) {
       err = cudaEventRecord(e0, own_stream);
       if (err == cudaSuccess)
-        err = brc::filter3d_fp32(tmp1.as<float>(), W, H, D, (int)nb, V, h_filters, nfilt, tmp2.as<float>(),
-                                 brc::all_instances(), own_stream, sym, cand[c]);
+        err = brc::filter3d_fp32(tmp1.as<float>(), W, H, D, nb, V, bank, kind, nfilt, tmp2.as<float>(),
+                                 brc::all_instances(), own_stream, cand[c]);
       if (err == cudaSuccess) err = cudaEventRecord(e1, own_stream);
       if (err == cudaSuccess) err = cudaEventSynchronize(e1);
       float ms = 0.f;
@@ -276,8 +275,11 @@ int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precis
   fp->nfilt = nfilt;
   fp->d_taps = nullptr;
   fp->d_err = ctx->tc_err.as<int>();
-  if (precision == BRC_PREC_FP32 || precision == BRC_PREC_FP32_GENERAL)
-    return ctx->tune_fp32(h_filters, nfilt, precision == BRC_PREC_FP32, W, H, D, batch, &fp->tz);
+  if (precision == BRC_PREC_FP32 || precision == BRC_PREC_FP32_GENERAL) {
+    // packed once for the tuner's key and every launch of this path
+    fp->kind = brc::filter3d_pack(h_filters, nfilt, precision == BRC_PREC_FP32, fp->bank);
+    return ctx->tune_fp32(fp->bank, fp->kind, nfilt, W, H, D, batch, &fp->tz);
+  }
   if (precision != BRC_PREC_BF16X3 && precision != BRC_PREC_TF32)
     return ctx->fail(BRC_ERR_UNSUPPORTED, "unknown precision");
   const bool tf32 = precision == BRC_PREC_TF32;
@@ -295,8 +297,7 @@ cudaError_t run_filter(const FilterPath& fp, const float* vol, int W, int H, int
   if (fp.precision == BRC_PREC_BF16X3 || fp.precision == BRC_PREC_TF32)
     return brc::tc::launch(vol, W, H, D, batch, stride, fp.d_taps, fp.nfilt, out, act, fp.d_err, fp.g, st,
                            fp.precision == BRC_PREC_TF32);
-  return brc::filter3d_fp32(vol, W, H, D, batch, stride, fp.h_filters, fp.nfilt, out, act, st,
-                            fp.precision == BRC_PREC_FP32, fp.tz);
+  return brc::filter3d_fp32(vol, W, H, D, batch, stride, fp.bank, fp.kind, fp.nfilt, out, act, st, fp.tz);
 }
 
 extern "C" {

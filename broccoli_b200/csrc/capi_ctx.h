@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "filter3d_tc.h"
+#include "internal.h"
 
 #include "../../include/broccoli_b200.h"
 
@@ -127,11 +128,10 @@ struct brc_ctx {
   // under capture the cost model's first choice).
   int tune_tc(int nfilt, int W, int H, int D, const uint16_t* d_taps, bool tf32, int* ty);
   // z depth of the FP32 filtering's output block for this shape, launch size
-  // and kind of kernel (even/odd when sym and the bank is symmetric, else
-  // general): the candidates timed once (outside stream capture), then
+  // and kind of kernel (of the packed bank): the candidates timed once (outside stream capture), then
   // cached.  Launch sizes count by powers of two: a launch that does not fill
   // the chip wants many small blocks, a large one few halos.
-  int tune_fp32(const float* h_filters, int nfilt, bool sym, int W, int H, int D, int batch, int* tz);
+  int tune_fp32(const float* bank, brc::FilterKind kind, int nfilt, int W, int H, int D, int batch, int* tz);
   // brc::smooth3d with the z chunk tuned per (shape, batch, certainty
   // kind): the first call of a key that writes a buffer it does not read
   // and does not accumulate (outside stream capture) runs every candidate
@@ -162,7 +162,10 @@ struct FilterPath {
   const uint16_t* d_taps = nullptr;
   brc::tc::Geometry g{};
   int* d_err = nullptr;
-  int tz = 0;  // FP32 filtering: z depth of the output block (0: untimed choice)
+  // FP32 filtering: the packed bank, its kind, and the z depth of the output block (0: untimed choice)
+  alignas(16) float bank[brc::kPackedBankFloats];
+  brc::FilterKind kind = brc::kFilterGeneral;
+  int tz = 0;
 };
 // batch: the volumes of the launches to come (any launch size is correct).
 int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precision, int W, int H, int D,

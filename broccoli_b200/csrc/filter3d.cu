@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "internal.h"
 
 namespace brc {
 
@@ -343,22 +344,26 @@ static inline float tap_weight(const float* h_filters, int k, int c, int dx, int
 }
 
 // True (and the symmetrised bank) when every filter of the bank has an even
-// real and odd imaginary part to 1e-6 of its largest tap.
+// real and odd imaginary part to 1e-6 of its largest tap.  Tap i of a filter
+// and its point reflection are i and 342 - i.
 template <int NF>
 static bool pack_sym_bank(const float* h_filters, SymBank<NF>& bank) {
   for (int k = 0; k < NF; k++) {
+    const float* f = h_filters + k * kFilterFloats;
+    float part[8] = {0.f};  // independent maxima: no chain of 686 compares
+    for (int i = 0; i < kFilterFloats; i++) {
+      const float v = fabsf(f[i]);
+      part[i & 7] = v > part[i & 7] ? v : part[i & 7];
+    }
     float mx = 0.f;
-    for (int i = 0; i < kFilterFloats; i++) mx = fmaxf(mx, fabsf(h_filters[k * kFilterFloats + i]));
+    for (int i = 0; i < 8; i++) mx = fmaxf(mx, part[i]);
     const float tol = 1e-6f * mx;
-    for (int dz = -3; dz <= 3; dz++)
-      for (int dy = -3; dy <= 3; dy++)
-        for (int dx = -3; dx <= 3; dx++) {
-          const float re = tap_weight(h_filters, k, 0, dx, dy, dz);
-          const float rm = tap_weight(h_filters, k, 0, -dx, -dy, -dz);
-          const float im = tap_weight(h_filters, k, 1, dx, dy, dz);
-          const float imm = tap_weight(h_filters, k, 1, -dx, -dy, -dz);
-          if (fabsf(re - rm) > tol || fabsf(im + imm) > tol) return false;
-        }
+    bool odd = false;
+    for (int i = 0; i <= kTaps / 2; i++) {
+      odd |= fabsf(f[i] - f[kTaps - 1 - i]) > tol;
+      odd |= fabsf(f[kTaps + i] + f[2 * kTaps - 1 - i]) > tol;
+    }
+    if (odd) return false;
   }
   auto put = [&](int slot, int dx, int dy, int dz) {
     for (int k = 0; k < NF; k++) {
@@ -457,18 +462,6 @@ int filter3d_tz_candidates(int* tz, int max_n) {
 
 int filter3d_default_tz(int D) { return pick_tz(D); }
 
-bool filter3d_bank_symmetric(const float* h_filters, int nfilt) {
-  if (nfilt == 3) {
-    SymBank<3> sb;
-    return pack_sym_bank<3>(h_filters, sb);
-  }
-  if (nfilt == 6) {
-    SymBank<6> sb;
-    return pack_sym_bank<6>(h_filters, sb);
-  }
-  return false;
-}
-
 template <typename Launch>
 static cudaError_t dispatch_tz(int tz, Launch launch) {
   switch (tz) {
@@ -481,39 +474,33 @@ static cudaError_t dispatch_tz(int tz, Launch launch) {
   }
 }
 
-cudaError_t filter3d_fp32(const float* vol, int W, int H, int D, int batch, long long stride,
-                          const float* h_filters, int nfilt, float* out, ActiveSet act, cudaStream_t st,
-                          bool allow_symmetric, int tz) {
-  if (tz <= 0) tz = pick_tz(D);
-  if (allow_symmetric && nfilt == 3) {
-    SymBank<3> sb;
-    if (pack_sym_bank<3>(h_filters, sb))
-      return dispatch_tz(tz, [&](auto T) {
-        return launch_sym<3, 8, decltype(T)::value>(vol, W, H, D, batch, stride, sb, out, act, st);
-      });
-  }
-  if (allow_symmetric && nfilt == 6) {
-    SymBank<6> sb;
-    if (pack_sym_bank<6>(h_filters, sb))
-      return dispatch_tz(tz, [&](auto T) {
-        return launch_sym<6, 4, decltype(T)::value>(vol, W, H, D, batch, stride, sb, out, act, st);
-      });
-  }
+FilterKind filter3d_pack(const float* h_filters, int nfilt, bool allow_symmetric, float* bank) {
   if (nfilt == 3) {
-    FilterBank<3> bank;
-    pack_bank<3>(h_filters, bank);
-    return dispatch_tz(tz, [&](auto T) {
-      return launch_fp32<3, 8, decltype(T)::value>(vol, W, H, D, batch, stride, bank, out, act, st);
-    });
+    if (allow_symmetric && pack_sym_bank<3>(h_filters, *reinterpret_cast<SymBank<3>*>(bank))) return kFilterSym;
+    pack_bank<3>(h_filters, *reinterpret_cast<FilterBank<3>*>(bank));
+  } else {
+    if (allow_symmetric && pack_sym_bank<6>(h_filters, *reinterpret_cast<SymBank<6>*>(bank))) return kFilterSym;
+    pack_bank<6>(h_filters, *reinterpret_cast<FilterBank<6>*>(bank));
   }
-  if (nfilt == 6) {
-    FilterBank<6> bank;
-    pack_bank<6>(h_filters, bank);
-    return dispatch_tz(tz, [&](auto T) {
-      return launch_fp32<6, 4, decltype(T)::value>(vol, W, H, D, batch, stride, bank, out, act, st);
-    });
-  }
-  return cudaErrorInvalidValue;
+  return kFilterGeneral;
+}
+
+cudaError_t filter3d_fp32(const float* vol, int W, int H, int D, int batch, long long stride, const float* bank,
+                          FilterKind kind, int nfilt, float* out, ActiveSet act, cudaStream_t st, int tz) {
+  if (tz <= 0) tz = pick_tz(D);
+  if (nfilt != 3 && nfilt != 6) return cudaErrorInvalidValue;
+  return dispatch_tz(tz, [&](auto T) {
+    constexpr int kTz = decltype(T)::value;
+    if (kind == kFilterSym)
+      return nfilt == 3 ? launch_sym<3, 8, kTz>(vol, W, H, D, batch, stride,
+                                                *reinterpret_cast<const SymBank<3>*>(bank), out, act, st)
+                        : launch_sym<6, 4, kTz>(vol, W, H, D, batch, stride,
+                                                *reinterpret_cast<const SymBank<6>*>(bank), out, act, st);
+    return nfilt == 3 ? launch_fp32<3, 8, kTz>(vol, W, H, D, batch, stride,
+                                               *reinterpret_cast<const FilterBank<3>*>(bank), out, act, st)
+                      : launch_fp32<6, 4, kTz>(vol, W, H, D, batch, stride,
+                                               *reinterpret_cast<const FilterBank<6>*>(bank), out, act, st);
+  });
 }
 
 }  // namespace brc
