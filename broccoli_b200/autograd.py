@@ -139,6 +139,41 @@ class Filter3d(torch.autograd.Function):
         return out, None
 
 
+class FilterSsd(torch.autograd.Function):
+    """Real volumes (B,D,H,W) and reference responses (B,nfilt,D,H,W,2) ->
+    sum of squared response differences."""
+
+    @staticmethod
+    def forward(fctx, vol, filters, q_ref):
+        c = _ctx(vol.device)
+        f = _host_filters(filters)
+        v = vol.contiguous()
+        B, D, H, W = v.shape
+        r = q_ref.detach().contiguous()
+        res = torch.empty_like(r)
+        loss = torch.empty((), dtype=torch.float32, device=v.device)
+        fn = _sig("brc_filter3d_ssd", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P])
+        _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), f.shape[0], _p(r), _p(res),
+                     _p(loss)))
+        fctx.filters = f
+        fctx.save_for_backward(res)
+        return loss
+
+    @staticmethod
+    def backward(fctx, g):
+        res, = fctx.saved_tensors
+        c = _ctx(res.device)
+        f = fctx.filters
+        B, nf, D, H, W, _ = res.shape
+        gl = g.contiguous().to(torch.float32)
+        gv = None
+        if fctx.needs_input_grad[0]:
+            gv = torch.empty((B, D, H, W), dtype=torch.float32, device=res.device)
+            fn = _sig("brc_filter3d_ssd_adjoint", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P])
+            _check(c, fn(c.handle, _p(res), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), nf, _p(gl), _p(gv)))
+        return gv, None, (-2.0 * gl) * res if fctx.needs_input_grad[2] else None
+
+
 def smooth3d(vol, sigma: float):
     return Smooth3d.apply(vol, gaussian_taps(sigma))
 
@@ -172,5 +207,10 @@ def registration_objective(moving: torch.Tensor, q_ref: torch.Tensor, filters, s
         w = warp_affine(s, params.reshape(1, 12))
     else:
         w = warp_field(s[0], field)[None]
+    # one fused pass where the reference responses have the responses' own
+    # layout; anything that broadcasts or converts goes through torch
+    if (isinstance(q_ref, torch.Tensor) and q_ref.dtype == torch.float32 and q_ref.device == w.device
+            and tuple(q_ref.shape) == (w.shape[0], len(filters)) + tuple(w.shape[1:]) + (2,)):
+        return FilterSsd.apply(w, filters, q_ref)
     q = filter3d(w, filters)
     return ((q - q_ref) ** 2).sum()

@@ -59,7 +59,8 @@ struct AdjBank {
 template <int NF>
 __global__ void __launch_bounds__(kAdjThreads, 3)
 filter3d_adjoint_kernel(const float* __restrict__ grad, int W, int H, int D,
-                        const __grid_constant__ AdjBank<NF> bank, float* __restrict__ out) {
+                        const __grid_constant__ AdjBank<NF> bank, float* __restrict__ out,
+                        const float* __restrict__ scale) {
   extern __shared__ __align__(16) F2 adj_smem[];
   F2* s_g = adj_smem;
   F2* s_w = adj_smem + kAdjSlices * kAdjSlice;
@@ -164,6 +165,7 @@ filter3d_adjoint_kernel(const float* __restrict__ grad, int W, int H, int D,
   }
   const int x0 = tile_x0 + kAdjR * tx, z = tile_z0 + tz;
   if (z >= D) return;
+  const float f = scale ? 2.0f * *scale : 1.0f;  // 1: the sum itself, bit for bit
 #pragma unroll
   for (int yy = 0; yy < kAdjY; yy++) {
     const int y = tile_y0 + kAdjY * yg + yy;
@@ -173,7 +175,7 @@ filter3d_adjoint_kernel(const float* __restrict__ grad, int W, int H, int D,
     for (int r = 0; r < kAdjR; r++)
       if (x0 + r < W) {
         const float2 v = f2_unpack(acc[yy][r]);
-        o[r] = v.x + v.y;
+        o[r] = f * (v.x + v.y);
       }
   }
 }
@@ -323,7 +325,7 @@ warp_field_backward_kernel(const float* __restrict__ src, int W, int H, int D, c
 
 template <int NF>
 static cudaError_t launch_adjoint(const float* grad, int W, int H, int D, int batch, const float* h_filters,
-                                  float* out, cudaStream_t st) {
+                                  float* out, const float* scale, cudaStream_t st) {
   AdjBank<NF> bank;
   for (int k = 0; k < NF; k++)
     for (int ez = -3; ez <= 3; ez++)
@@ -345,15 +347,85 @@ static cudaError_t launch_adjoint(const float* grad, int W, int H, int D, int ba
   }
   const int z_tiles = (D + kAdjTZ - 1) / kAdjTZ;
   dim3 grid((W + kAdjTX - 1) / kAdjTX, ((H + kAdjTY - 1) / kAdjTY) * z_tiles, batch);
-  filter3d_adjoint_kernel<NF><<<grid, kAdjThreads, kAdjSmem, st>>>(grad, W, H, D, bank, out);
+  filter3d_adjoint_kernel<NF><<<grid, kAdjThreads, kAdjSmem, st>>>(grad, W, H, D, bank, out, scale);
   return cudaGetLastError();
 }
 
 cudaError_t filter3d_adjoint(const float* grad, int W, int H, int D, int batch, const float* h_filters, int nfilt,
-                             float* out, cudaStream_t st) {
-  if (nfilt == 3) return launch_adjoint<3>(grad, W, H, D, batch, h_filters, out, st);
-  if (nfilt == 6) return launch_adjoint<6>(grad, W, H, D, batch, h_filters, out, st);
+                             float* out, cudaStream_t st, const float* scale) {
+  if (nfilt == 3) return launch_adjoint<3>(grad, W, H, D, batch, h_filters, out, scale, st);
+  if (nfilt == 6) return launch_adjoint<6>(grad, W, H, D, batch, h_filters, out, scale, st);
   return cudaErrorInvalidValue;
+}
+
+// Sum of squared differences.  q becomes q - ref in place (the backward pass
+// needs the difference, and 2 g times it goes through the adjoint filtering
+// as a factor of its output), and each block writes the FP64 sum of its
+// squares; sum_partials_kernel adds the blocks in order.  Bound by memory:
+// two reads and a write per value, one pass where subtraction, square, sum and
+// their backward products were six (128x128x96, three filters: objective and
+// gradient 432 -> 367 us).
+constexpr int kSsdThreads = 256, kSsdBlocks = 148 * 8;
+
+template <bool VEC>
+__global__ void __launch_bounds__(kSsdThreads)
+ssd_residual_kernel(float* __restrict__ q, const float* __restrict__ ref, long long n, double* __restrict__ partials) {
+  double sum = 0.0;
+  const long long step = (long long)gridDim.x * kSsdThreads;
+  const long long i0 = (long long)blockIdx.x * kSsdThreads + threadIdx.x;
+  if (VEC) {
+    float4* q4 = reinterpret_cast<float4*>(q);
+    const float4* r4 = reinterpret_cast<const float4*>(ref);
+#pragma unroll 4
+    for (long long i = i0; i < n / 4; i += step) {
+      const float4 a = q4[i], b = __ldg(r4 + i);
+      const float4 d = make_float4(a.x - b.x, a.y - b.y, a.z - b.z, a.w - b.w);
+      q4[i] = d;
+      sum += (double)(d.x * d.x + d.y * d.y + d.z * d.z + d.w * d.w);
+    }
+  } else {
+    for (long long i = i0; i < n; i += step) {
+      const float d = q[i] - __ldg(ref + i);
+      q[i] = d;
+      sum += (double)(d * d);
+    }
+  }
+  __shared__ double s[kSsdThreads / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < kSsdThreads / 32; w++) sum += s[w];
+    partials[blockIdx.x] = sum;
+  }
+}
+
+// *out = sum of n partial sums (one warp, a fixed order).
+__global__ void sum_partials_kernel(const double* __restrict__ partials, int n, float* __restrict__ out) {
+  double v = 0.0;
+#pragma unroll 4
+  for (int r = threadIdx.x; r < n; r += 32) v += partials[r];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if (threadIdx.x == 0) *out = (float)v;
+}
+
+int ssd_blocks(long long n) {
+  const long long b = (n / 4 + kSsdThreads) / kSsdThreads;
+  return (int)(b < kSsdBlocks ? b : kSsdBlocks);
+}
+
+cudaError_t ssd_residual(float* q, const float* ref, long long n, double* partials, float* out, cudaStream_t st) {
+  const int nb = ssd_blocks(n);
+  // 16-byte accesses where both arrays allow them and no value is left over
+  if ((n & 3) == 0 && ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(ref)) & 15) == 0)
+    ssd_residual_kernel<true><<<nb, kSsdThreads, 0, st>>>(q, ref, n, partials);
+  else
+    ssd_residual_kernel<false><<<nb, kSsdThreads, 0, st>>>(q, ref, n, partials);
+  sum_partials_kernel<<<1, 32, 0, st>>>(partials, nb, out);
+  return cudaGetLastError();
 }
 
 int warp_affine_backward_blocks(long long V) {

@@ -812,6 +812,35 @@ extern "C" int brc_filter3d_adjoint(brc_ctx* ctx, const float* d_grad, int W, in
   return BRC_OK;
 }
 
+extern "C" int brc_filter3d_ssd(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch,
+                                const float* h_filters, int nfilt, const float* d_ref, float* d_residual,
+                                float* d_loss) {
+  if (!ctx) return BRC_ERR_INVALID;
+  if (!d_ref || !d_residual || !d_loss || d_ref == d_residual)
+    return ctx->fail(BRC_ERR_INVALID, "brc_filter3d_ssd: bad argument");
+  const int s = brc_filter3d(ctx, d_vol, W, H, D, batch, (long long)W * H * D, h_filters, nfilt, BRC_PREC_FP32,
+                             d_residual);
+  if (s != BRC_OK) return s;
+  const long long n = 2ll * nfilt * W * H * D * batch;
+  BRC_TRY(ctx, ctx->partials.ensure(sizeof(double) * (size_t)brc::ssd_blocks(n)), "alloc");
+  BRC_TRY(ctx, brc::ssd_residual(d_residual, d_ref, n, ctx->partials.as<double>(), d_loss, ctx->stream()), "ssd");
+  ctx->launches += 2;
+  return BRC_OK;
+}
+
+extern "C" int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, int W, int H, int D, int batch,
+                                        const float* h_filters, int nfilt, const float* d_grad_loss, float* d_out) {
+  if (!ctx) return BRC_ERR_INVALID;
+  if (!d_residual || !d_out || !h_filters || !d_grad_loss || W <= 0 || H <= 0 || D <= 0 || batch <= 0 ||
+      batch > 65535 || (nfilt != 3 && nfilt != 6))
+    return ctx->fail(BRC_ERR_INVALID, "brc_filter3d_ssd_adjoint: bad argument");
+  cudaSetDevice(ctx->device);
+  BRC_TRY(ctx, brc::filter3d_adjoint(d_residual, W, H, D, batch, h_filters, nfilt, d_out, ctx->stream(), d_grad_loss),
+          "filter3d_adjoint");
+  ctx->launches += 1;
+  return BRC_OK;
+}
+
 extern "C" int brc_warp_affine_backward(brc_ctx* ctx, const float* d_src, int W, int H, int D, int batch,
                                         const float* d_params, const float* d_grad_out, double* d_grad_params,
                                         float* d_grad_src) {

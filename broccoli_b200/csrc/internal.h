@@ -130,8 +130,12 @@ void host_invert_affine(const float* p12, float* inv12);
 
 namespace brc {
 // adjoint.cu
+// scale (device, may be null): the output is multiplied by 2 *scale.
 cudaError_t filter3d_adjoint(const float* grad, int W, int H, int D, int batch, const float* h_filters, int nfilt,
-                             float* out, cudaStream_t st);
+                             float* out, cudaStream_t st, const float* scale = nullptr);
+// q -= ref in place, *out = the sum of the squares; partials: ssd_blocks(n) doubles.
+int ssd_blocks(long long n);
+cudaError_t ssd_residual(float* q, const float* ref, long long n, double* partials, float* out, cudaStream_t st);
 int warp_affine_backward_blocks(long long V);
 cudaError_t warp_affine_backward(const float* src, int W, int H, int D, int batch, const float* params,
                                  const float* gout, double* partials, int nblk, double* gparams, float* gsrc,

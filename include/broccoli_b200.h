@@ -304,6 +304,17 @@ int brc_register_nonlinear(brc_ctx* ctx, const float* d_ref, const float* d_movi
 int brc_filter3d_adjoint(brc_ctx* ctx, const float* d_grad, int W, int H, int D, int batch,
                          const float* h_filters, int nfilt, float* d_out);
 
+/* The objective of the differentiable registration in one call: the FP32
+ * responses of d_vol (as brc_filter3d) minus the reference responses d_ref
+ * (the same layout) into d_residual, and the sum of the squares into d_loss
+ * (one float).  brc_filter3d_ssd_adjoint is its adjoint: d_out = dL/dvol =
+ * 2 *d_grad_loss times the adjoint filtering of the residual (d_grad_loss one
+ * device float, dL/dloss).  No counterpart in the reference. */
+int brc_filter3d_ssd(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch, const float* h_filters,
+                     int nfilt, const float* d_ref, float* d_residual, float* d_loss);
+int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, int W, int H, int D, int batch,
+                             const float* h_filters, int nfilt, const float* d_grad_loss, float* d_out);
+
 /* Adjoint of brc_warp_affine: dL/dparams (batch x 12, double) from the
  * output gradient, with the exact derivative of the clamp-to-edge
  * trilinear interpolant; d_grad_src (may be NULL) receives dL/dsrc by
