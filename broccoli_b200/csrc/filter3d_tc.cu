@@ -45,11 +45,11 @@
 //   warps 12-19    stage a tile's input (FP32 -> BF16 hi/lo or TF32 rows)
 //                  into one of two shared-memory buffers while the GEMMs
 //                  read the other
-//   warp 1, lane 0 issues the tcgen05.mma's: three split products (BF16X3)
+//   warp 1         issues the tcgen05.mma's from an elected lane: three split products (BF16X3)
 //                  or one sparse MMA (TF32) per stage, descriptors built
 //                  once and advanced by adds (every cycle of address
 //                  arithmetic in this thread delays the GEMMs)
-//   warp 2, lane 0 streams the packed taps, two stages (BF16X3: 16 KB, hi
+//   warp 2         streams the packed taps (one elected lane), two stages (BF16X3: 16 KB, hi
 //                  + lo of each; TF32: 8 KB) per slot, through a 3-slot
 //                  ring with cp.async.bulk + mbarriers (one wait and one
 //                  commit per two GEMMs)
@@ -77,16 +77,15 @@
 namespace brc {
 namespace tc {
 
-// Group sizes measured on 199 volumes of 64x64x33 (dense TF32 / BF16X3 ms):
-// 4 + 4 warps 0.58 / 0.72, 8 + 4 0.57 / 0.74, 4 + 8 0.66 / 0.72, 8 + 8
-// 0.534 / 0.696, 12 + 8 and 8 + 12 0.54-0.55 / 0.70.
+// Group sizes measured on 199 volumes of 64x64x33 (TF32, epilogue + staging
+// warps): 8 + 8 357 us, 8 + 4 404, 8 + 12 385, 4 + 8 377.
 constexpr int kEpiWarps = 8;         // epilogue warps (a multiple of 4: kEpiWarps / 4 per TMEM lane quarter)
 constexpr int kStageWarps = 8;       // staging warps
 constexpr int kStageWarp = 4 + kEpiWarps;                    // first staging warp
 constexpr int kThreads = 32 * (4 + kEpiWarps + kStageWarps);  // roles above
 constexpr int kEpiThreads = 32 * kEpiWarps, kStageThreads = 32 * kStageWarps;
 constexpr int kEpiGroups = kEpiThreads / 30;  // accumulator columns stored at once (30 pieces each)
-constexpr int kRing = 3;             // tap slots in flight (two stages each; 2, 4, 5, 6 measured slower)
+constexpr int kRing = 3;             // tap slots in flight (two stages each; TF32: 2 426 us, 4 386, 6 447)
 constexpr int kEpiCols = 64;         // accumulator columns per epilogue chunk
 constexpr uint32_t kTmemCols = 512;  // two accumulators of up to 256 columns
 constexpr int kStageHalves = kM * kK;              // BF16 elements of one A (hi or lo)
@@ -168,6 +167,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return true;
 }
 
+// mbar_wait by a whole warp: true on every lane or on none.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity)) != 0;
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P1;\n\t"
+      "elect.sync _|P1, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, P1;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
@@ -203,9 +218,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Named barriers of the 128-thread groups (0 is __syncthreads).
+// Named barrier of the epilogue threads (0 is __syncthreads).
 __device__ __forceinline__ void epi_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory"); }
-__device__ __forceinline__ void stage_sync() { asm volatile("bar.sync 2, %0;" ::"n"(kStageThreads) : "memory"); }
 
 struct TileArgs {
   long long vstride;       // floats between volumes
@@ -215,6 +229,7 @@ struct TileArgs {
   uint32_t in_off;         // shared offsets: input buffers, epilogue buffer, barriers
   uint32_t e_off;
   uint32_t bar_off;
+  uint32_t tab_off;
 };
 
 // Tile t of the launch -> (instance b, zt, yt, xc), xc fastest; the
@@ -282,12 +297,33 @@ __device__ __forceinline__ uint32_t tf32_rna(float x) {
   return r;
 }
 
+// A staged row on its way from global to shared memory: the aligned quads
+// that cover its 16 samples, the position of sample 0 in them, its x
+// coordinate and the row's byte offset in the buffer (-1: no row).
+struct RowRegs {
+  float4 f[5];
+  int al, xs, off;
+};
+
+// The aligned quad at p, of which at least one element is inside [beg, end):
+// elements outside are not read.
+__device__ __forceinline__ float4 load_quad(const float* p, const float* beg, const float* end) {
+  if (p >= beg && p + 4 <= end) return __ldg(reinterpret_cast<const float4*>(p));
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p >= beg && p < end) v.x = __ldg(p);
+  if (p + 1 >= beg && p + 1 < end) v.y = __ldg(p + 1);
+  if (p + 2 >= beg && p + 2 < end) v.z = __ldg(p + 2);
+  if (p + 3 >= beg && p + 3 < end) v.w = __ldg(p + 3);
+  return v;
+}
+
 template <bool TF32>
 __global__ void __launch_bounds__(kThreads, 1)
 filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ taps, float* __restrict__ out,
                    const TileArgs a, const Geometry g, const ActiveSet act, int* __restrict__ err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // the same for the compiler too
   uint8_t* ring = smem;
   uint8_t* inb = smem + a.in_off;
   float* E = reinterpret_cast<float*>(smem + a.e_off);
@@ -300,14 +336,24 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
   uint64_t* done = tempty + kRing;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   // [1] tiles the GEMMs finished, [2] tap stages loaded, [3] tap stages
-  // consumed, [4] a wait gave up, [5] / [6] epilogue / staging broadcasts
+  // consumed, [4] a wait gave up, [5] the epilogue's broadcast
   int* flags = reinterpret_cast<int*>(tmem_slot + 1);
 
   // one K half of one part (hi or lo) of one input buffer: NR 16-byte rows
   const uint32_t rowbytes = 16u * (uint32_t)g.NR;
   const long long V = (long long)a.W * a.H * a.D;
+  const int prow = a.nqp * g.Hp;   // staged rows per parity array
+  const int nrows = g.SP * prow;   // staged rows of a tile
+  // row -> (plane offset | y offset << 16, byte offset in the buffer)
+  uint2* rowtab = reinterpret_cast<uint2*>(smem + a.tab_off);
+  for (int row = tid; row < nrows; row += kThreads) {
+    const int par = row / prow, rr = row - par * prow;
+    const int qq = rr / g.Hp, yl = rr - qq * g.Hp;
+    rowtab[row] = make_uint2((uint32_t)(qq * g.SP + par) | ((uint32_t)yl << 16),
+                             (uint32_t)(par * g.RP + qq * g.Hp + yl) * 16u);
+  }
   // every role walks the same tiles: those of the active instances
-  const int ntiles = active_count(act, a.batch) * a.tiles_per;
+  const int ntiles = __shfl_sync(0xffffffffu, active_count(act, a.batch) * a.tiles_per, 0);
 
   if (tid == 0) {
     for (int i = 0; i < 2; i++) {
@@ -333,7 +379,7 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   if (TF32) {
     // the sparsity metadata, one column for every MMA of the launch
     if (warp >= 4 && warp < 8) {
@@ -351,122 +397,150 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
   }
 
   if (warp >= kStageWarp) {
-    // ---- staging: row (parity p, plane slot qq, y row yl) of K half kh
-    // holds the 8 samples x0-3+8kh .. x0+4+8kh of input plane z0-3+SP*qq+p,
-    // row y0-3+yl (zero outside the volume), as BF16 hi and lo.
+    // ---- staging: row (parity p, plane slot qq, y row yl) holds the 16
+    // samples x0-3 .. x0+12 of input plane z0-3+SP*qq+p, row y0-3+yl (zero
+    // outside the volume), as two K halves of BF16 hi and lo or in the K order
+    // of the sparse TF32 MMA.  A thread takes every kStageThreads-th row of a
+    // tile and keeps the loads of two rows in flight, across tiles too: the
+    // loads of the next tile's first rows are issued before this thread waits
+    // for that tile's buffer.  (199 volumes of 64x64x33: 375 -> 357 us; six
+    // filters at 182x218x182, whose rows are not 16-byte aligned and were
+    // loaded one sample at a time: 173 -> 168 us.  Neither is bound by one
+    // role now: without the staging's loads, the stores, the tap copies or with
+    // N = 16 the launch takes 80-87 % of its time.)
     const int st = tid - kStageWarp * 32;
-    const int prow = a.nqp * g.Hp;   // staged rows per parity array
-    const int nrows = g.SP * prow;   // staged rows per K half
-    int i = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-      int b, zt, yt, xc;
-      decode_tile(a, act, t, b, zt, yt, xc);
-      const int buf = i & 1;
-      // one thread waits for the buffer and tells the others
-      if (st == 0) flags[6] = (i < 2 || mbar_wait(&empty_in[buf], (uint32_t)((i >> 1) - 1) & 1u)) ? 1 : 0;
-      stage_sync();
-      const bool go = *reinterpret_cast<volatile int*>(&flags[6]) != 0;
-      stage_sync();
-      if (!go) {
-        ok = false;
-        break;
+    const int nit = (nrows + kStageThreads - 1) / kStageThreads;
+    const float* const vbeg = vol;
+    const float* const vend = vol + (long long)(a.batch - 1) * a.vstride + V;
+    // all rows 16-byte aligned: the window offset is 1 or 3 for a whole tile
+    const bool aligned = (a.W & 3) == 0 && (reinterpret_cast<uintptr_t>(vol) & 15) == 0 && (a.vstride & 3) == 0;
+    int lt = blockIdx.x, lit = 0;  // load cursor: tile and row of this thread
+    int lx = 0, ly = 0, lz = 0;
+    const float* lsrc = vol;
+    auto seek = [&]() {
+      if (lt < ntiles) {
+        int b, zt, yt, xc;
+        decode_tile(a, act, lt, b, zt, yt, xc);
+        lx = xc * kXo - 3;
+        ly = yt * g.Ty - 3;
+        lz = zt * g.SP * g.J - 3;
+        lsrc = vol + (long long)b * a.vstride;
       }
-      const int x0 = xc * kXo, y0 = yt * g.Ty, z0 = zt * g.SP * g.J;
-      const float* src = vol + (long long)b * a.vstride;
-      // rows are 16-byte aligned when W is a multiple of 4 (and the volume
-      // is): a window inside the row then takes three aligned float4 loads
-      const bool vec_rows = (a.W & 3) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-      uint8_t* hi = inb + (uint32_t)(buf * 4) * rowbytes;
-      uint8_t* lo = hi + 2u * rowbytes;
-      if (TF32) {
-        // whole rows of 16 samples x0 - 3 .. x0 + 12, in the K order of the
-        // sparse MMA: quarter q holds samples 2q, 2q + 8, 2q + 1, 2q + 9
-        for (int row = st; row < nrows; row += kStageThreads) {
-          const int par = row / prow, rr = row - par * prow;
-          const int qq = rr / g.Hp, yl = rr - qq * g.Hp;
-          const int zg = z0 - 3 + qq * g.SP + par, yg = y0 - 3 + yl;
-          const bool rowok = zg >= 0 && zg < a.D && yg >= 0 && yg < a.H;
-          const int xs = x0 - 3;
-          float v[16];
-          if (rowok && vec_rows && xs >= 0 && (xs & ~3) + 20 <= a.W) {
-            const int al = xs & 3;
-            const float4* p4 = reinterpret_cast<const float4*>(src + ((long long)zg * a.H + yg) * a.W + (xs - al));
-            const float4 f0 = __ldg(p4), f1 = __ldg(p4 + 1), f2 = __ldg(p4 + 2), f3 = __ldg(p4 + 3),
-                         f4 = __ldg(p4 + 4);
-            const float w[20] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y,
-                                 f2.z, f2.w, f3.x, f3.y, f3.z, f3.w, f4.x, f4.y, f4.z, f4.w};
-#pragma unroll
-            for (int e = 0; e < 16; e++)
-              v[e] = al == 0 ? w[e] : (al == 1 ? w[e + 1] : (al == 2 ? w[e + 2] : w[e + 3]));
-          } else {
-            const float* rp = src + ((long long)(rowok ? zg : 0) * a.H + (rowok ? yg : 0)) * a.W;
-#pragma unroll
-            for (int e = 0; e < 16; e++) {
-              const int xg = xs + e;
-              v[e] = (rowok && xg >= 0 && xg < a.W) ? __ldg(rp + xg) : 0.f;
-            }
-          }
-          const uint32_t rowoff = (uint32_t)(par * g.RP + qq * g.Hp + yl) * 16u;
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            *reinterpret_cast<uint4*>(hi + (uint32_t)q * rowbytes + rowoff) =
-                make_uint4(tf32_rna(v[2 * q]), tf32_rna(v[2 * q + 8]), tf32_rna(v[2 * q + 1]), tf32_rna(v[2 * q + 9]));
-        }
-      }
-      for (int item = st; !TF32 && item < 2 * nrows; item += kStageThreads) {
-        const int kh = item >= nrows ? 1 : 0, row = item - kh * nrows;
-        const int par = row / prow, rr = row - par * prow;
-        const int qq = rr / g.Hp, yl = rr - qq * g.Hp;
-        const int zg = z0 - 3 + qq * g.SP + par, yg = y0 - 3 + yl;
+    };
+    seek();
+    auto fetch = [&](RowRegs& r) {
+      r.off = -1;
+      if (lt >= ntiles) return;
+      const int row = st + lit * kStageThreads;
+      if (row < nrows) {
+        const uint2 e = rowtab[row];
+        const int zg = lz + (int)(e.x & 0xffffu), yg = ly + (int)(e.x >> 16);
+        r.off = (int)e.y;
+        r.xs = lx;
+        const float* p = lsrc + ((long long)zg * a.H + yg) * a.W + lx;  // sample 0 (maybe outside the row)
+        const int al = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3);
+        r.al = al;
         const bool rowok = zg >= 0 && zg < a.D && yg >= 0 && yg < a.H;
-        const int xs = x0 - 3 + 8 * kh;
-        float v[8];
-        if (rowok && vec_rows && xs >= 0 && (xs & ~3) + 12 <= a.W) {
-          const int al = xs & 3;
-          const float4* p4 = reinterpret_cast<const float4*>(src + ((long long)zg * a.H + yg) * a.W + (xs - al));
-          const float4 f0 = __ldg(p4), f1 = __ldg(p4 + 1), f2 = __ldg(p4 + 2);
-          const float w[12] = {f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w, f2.x, f2.y, f2.z, f2.w};
+        // aligned quads that hold a sample of this window inside the row
+        const int lo = lx > 0 ? lx : 0, hi = lx + 16 < a.W ? lx + 16 : a.W;
 #pragma unroll
-          for (int e = 0; e < 8; e++) v[e] = al == 0 ? w[e] : (al == 1 ? w[e + 1] : (al == 2 ? w[e + 2] : w[e + 3]));
-        } else {
-          const float* rp = src + ((long long)(rowok ? zg : 0) * a.H + (rowok ? yg : 0)) * a.W;
-#pragma unroll
-          for (int e = 0; e < 8; e++) {
-            const int xg = xs + e;
-            v[e] = (rowok && xg >= 0 && xg < a.W) ? __ldg(rp + xg) : 0.f;
-          }
+        for (int k = 0; k < 5; k++) {
+          const int c = lx - al + 4 * k;
+          r.f[k] = rowok && c + 3 >= lo && c < hi ? load_quad(p - al + 4 * k, vbeg, vend)
+                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        const uint32_t rowoff = (uint32_t)(par * g.RP + qq * g.Hp + yl) * 16u;
-        {
+      }
+      if (++lit == nit) {
+        lit = 0;
+        lt += gridDim.x;
+        seek();
+      }
+    };
+    auto put = [&](const RowRegs& r, uint8_t* hi) {
+      if (r.off < 0) return;
+      const float w[20] = {r.f[0].x, r.f[0].y, r.f[0].z, r.f[0].w, r.f[1].x, r.f[1].y, r.f[1].z,
+                           r.f[1].w, r.f[2].x, r.f[2].y, r.f[2].z, r.f[2].w, r.f[3].x, r.f[3].y,
+                           r.f[3].z, r.f[3].w, r.f[4].x, r.f[4].y, r.f[4].z, r.f[4].w};
+      float v[16];
+      if (aligned) {
+#pragma unroll
+        for (int e = 0; e < 16; e++) v[e] = (r.al & 2) ? w[e + 3] : w[e + 1];
+      } else {
+        float h[17];
+#pragma unroll
+        for (int e = 0; e < 17; e++) h[e] = (r.al & 2) ? w[e + 2] : w[e];
+#pragma unroll
+        for (int e = 0; e < 16; e++) v[e] = (r.al & 1) ? h[e + 1] : h[e];
+        // quads of an unaligned row may reach into its neighbours
+        if (r.xs < 0 || r.xs + 16 > a.W) {
+#pragma unroll
+          for (int e = 0; e < 16; e++) v[e] = (unsigned)(r.xs + e) < (unsigned)a.W ? v[e] : 0.f;
+        }
+      }
+      uint8_t* d = hi + r.off;
+      if (TF32) {
+        // quarter q holds samples 2q, 2q + 8, 2q + 1, 2q + 9
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+          *reinterpret_cast<uint4*>(d + (uint32_t)q * rowbytes) =
+              make_uint4(tf32_rna(v[2 * q]), tf32_rna(v[2 * q + 8]), tf32_rna(v[2 * q + 1]), tf32_rna(v[2 * q + 9]));
+      } else {
+#pragma unroll
+        for (int kh = 0; kh < 2; kh++) {
           uint32_t ph4[4], pl4[4];
 #pragma unroll
           for (int e = 0; e < 8; e += 2) {
-            const __nv_bfloat16 h0 = __float2bfloat16_rn(v[e]), h1 = __float2bfloat16_rn(v[e + 1]);
-            const __nv_bfloat16 l0 = __float2bfloat16_rn(v[e] - __bfloat162float(h0));
-            const __nv_bfloat16 l1 = __float2bfloat16_rn(v[e + 1] - __bfloat162float(h1));
+            const float v0 = v[8 * kh + e], v1 = v[8 * kh + e + 1];
+            const __nv_bfloat16 h0 = __float2bfloat16_rn(v0), h1 = __float2bfloat16_rn(v1);
+            const __nv_bfloat16 l0 = __float2bfloat16_rn(v0 - __bfloat162float(h0));
+            const __nv_bfloat16 l1 = __float2bfloat16_rn(v1 - __bfloat162float(h1));
             ph4[e / 2] = pack_bf16(h0, h1);
             pl4[e / 2] = pack_bf16(l0, l1);
           }
-          const uint32_t off = (uint32_t)kh * rowbytes + rowoff;
-          *reinterpret_cast<uint4*>(hi + off) = make_uint4(ph4[0], ph4[1], ph4[2], ph4[3]);
-          *reinterpret_cast<uint4*>(lo + off) = make_uint4(pl4[0], pl4[1], pl4[2], pl4[3]);
+          *reinterpret_cast<uint4*>(d + (uint32_t)kh * rowbytes) = make_uint4(ph4[0], ph4[1], ph4[2], ph4[3]);
+          *reinterpret_cast<uint4*>(d + (uint32_t)(kh + 2) * rowbytes) = make_uint4(pl4[0], pl4[1], pl4[2], pl4[3]);
         }
+      }
+    };
+    RowRegs ra, rb;
+    fetch(ra);
+    fetch(rb);
+    bool second = false;
+    int i = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
+      const int buf = i & 1;
+      if (i >= 2 && !mbar_wait(&empty_in[buf], (uint32_t)((i >> 1) - 1) & 1u)) {
+        flags[4] = 1;
+        break;
+      }
+      uint8_t* hi = inb + (uint32_t)(buf * 4) * rowbytes;
+      for (int it = 0; it < nit; it++) {
+        if (second) {
+          put(rb, hi);
+          fetch(rb);
+        } else {
+          put(ra, hi);
+          fetch(ra);
+        }
+        second = !second;
       }
       // the GEMMs read the buffer through the async proxy
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_arrive(&full_in[buf]);
-      i++;
     }
-    if (!ok) flags[4] = 1;
-  } else if (warp == 1 && lane == 0) {
-    // ---- GEMM issue.  The descriptors are built once; a stage only adds
-    // offsets to their start-address fields (one 16-byte row = 1), so that
-    // the issuing thread spends its time in tcgen05.mma, not in address
-    // arithmetic (which delays every GEMM it precedes).
+  } else if (warp == 1) {
+    // ---- GEMM issue.  The whole warp walks the loop and one elected lane
+    // issues: the descriptors then live in uniform registers, which the MMA
+    // reads directly.  (Computed by a single lane they were moved there for
+    // every MMA, which took 186 cycles each whatever N, 505 per ring slot of
+    // two sparse MMAs, and bounded the TF32 launch: with N = 16 in place of
+    // 224 it took 400 of its 416 us; the elected lane took it to 375 us for 199
+    // volumes of 64x64x33.)  The descriptors are built once; a stage
+    // only adds offsets to their start-address fields (one 16-byte row = 1).
     // D F32; A, B BF16 (1) or TF32 (2); K-major; N, M
     // (TF32: structured-sparse MMAs, sparse flag bit 2, metadata in TMEM
     // column kMetaCol)
+    const bool leader = elect_one();
     const uint32_t ab = TF32 ? 2u : 1u;
     const uint32_t idesc = (TF32 ? (1u << 2) : 0u) | (1u << 4) | (ab << 7) | (ab << 10) |
                            ((uint32_t)(g.N >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
@@ -492,11 +566,9 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
     uint64_t ah = da0;
     bool ok = true;
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      int b, zt, yt, xc;
-      decode_tile(a, act, t, b, zt, yt, xc);
       const int buf = i & 1, acc = i & 1;
-      if (!mbar_wait(&full_in[buf], (uint32_t)(i >> 1) & 1u) ||
-          (i >= 2 && !mbar_wait(&acc_empty[acc], (uint32_t)((i >> 1) - 1) & 1u))) {
+      if (!mbar_wait_warp(&full_in[buf], (uint32_t)(i >> 1) & 1u) ||
+          (i >= 2 && !mbar_wait_warp(&acc_empty[acc], (uint32_t)((i >> 1) - 1) & 1u))) {
         ok = false;
         break;
       }
@@ -507,30 +579,33 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
       for (int dyq = 0; dyq < 7 && ok; dyq++) {
 #pragma unroll
         for (int m = 0; m < 4; m++) {
-          if (!mbar_wait(&tfull[slot], ph)) {
+          if (!mbar_wait_warp(&tfull[slot], ph)) {
             ok = false;
             break;
           }
           const uint64_t b1 = bh0 + offa[m] + (uint64_t)dyq;
-          if (TF32) {
-            mma_tf32_sp(dcol, ah, b1, tmem_e, idesc, accf);
-          } else {
-            mma_bf16(dcol, ah, b1, idesc, accf);
-            mma_bf16(dcol, ah, b1 + dblo, idesc, 1u);
-            mma_bf16(dcol, ah + dalo, b1, idesc, 1u);
-          }
-          accf = 1u;
-          if (m < 3 || last_pair) {
-            const uint64_t b2 = bh0 + offb[m] + (uint64_t)dyq, a2 = ah + dstage;
+          const uint64_t b2 = bh0 + offb[m] + (uint64_t)dyq, a2 = ah + dstage;
+          if (leader) {
             if (TF32) {
-              mma_tf32_sp(dcol, a2, b2, tmem_e, idesc, 1u);
+              mma_tf32_sp(dcol, ah, b1, tmem_e, idesc, accf);
             } else {
-              mma_bf16(dcol, a2, b2, idesc, 1u);
-              mma_bf16(dcol, a2, b2 + dblo, idesc, 1u);
-              mma_bf16(dcol, a2 + dalo, b2, idesc, 1u);
+              mma_bf16(dcol, ah, b1, idesc, accf);
+              mma_bf16(dcol, ah, b1 + dblo, idesc, 1u);
+              mma_bf16(dcol, ah + dalo, b1, idesc, 1u);
             }
+            if (m < 3 || last_pair) {
+              if (TF32) {
+                mma_tf32_sp(dcol, a2, b2, tmem_e, idesc, 1u);
+              } else {
+                mma_bf16(dcol, a2, b2, idesc, 1u);
+                mma_bf16(dcol, a2, b2 + dblo, idesc, 1u);
+                mma_bf16(dcol, a2 + dalo, b2, idesc, 1u);
+              }
+            }
+            mma_commit(&tempty[slot]);
           }
-          mma_commit(&tempty[slot]);
+          __syncwarp();
+          accf = 1u;
           G++;
           ah += dslot;
           if (++slot == kRing) {
@@ -541,36 +616,44 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
         }
       }
       if (!ok) break;
-      mma_commit(&empty_in[buf]);
-      mma_commit(&acc_full[acc]);
+      if (leader) {
+        mma_commit(&empty_in[buf]);
+        mma_commit(&acc_full[acc]);
+      }
+      __syncwarp();
       i++;
     }
-    flags[1] = i;
-    flags[3] = (int)G;
-    if (!ok) flags[4] = 1;
-    // on every exit, the give-up path included: one commit that tracks all
-    // MMAs this thread issued, waited on (bounded) before the TMEM and the
-    // shared-memory stages are released below
-    mma_commit(done);
-    if (!mbar_wait(done, 0)) flags[4] = 1;
-  } else if (warp == 2 && lane == 0) {
-    // ---- tap stages
+    if (leader) {
+      flags[1] = i;
+      flags[3] = (int)G;
+      if (!ok) flags[4] = 1;
+      // on every exit, the give-up path included: one commit that tracks all
+      // MMAs this thread issued, waited on (bounded) before the TMEM and the
+      // shared-memory stages are released below
+      mma_commit(done);
+      if (!mbar_wait(done, 0)) flags[4] = 1;
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // ---- tap stages (the warp waits, one elected lane copies)
+    const bool leader = elect_one();
     uint32_t G = 0, ph = 0;
     int slot = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      int b, zt, yt, xc;
-      decode_tile(a, act, t, b, zt, yt, xc);
       const uint16_t* src = taps;
       for (int s = 0; s < kSlotsPerTile; s++, G++) {
         // the slot's previous pair (G - kRing) must have been consumed
-        if (G >= (uint32_t)kRing && !mbar_wait(&tempty[slot], ph ^ 1u)) {
+        if (G >= (uint32_t)kRing && !mbar_wait_warp(&tempty[slot], ph ^ 1u)) {
           ok = false;
           break;
         }
         constexpr int kSl = TF32 ? kSlotBytesSp : kSlotBytes;
-        mbar_expect_tx(&tfull[slot], kSl);
-        bulk_load(ring + slot * kSl, src, kSl, &tfull[slot]);
+        if (leader) {
+          mbar_expect_tx(&tfull[slot], kSl);
+          bulk_load(ring + slot * kSl, src, kSl, &tfull[slot]);
+        }
+        __syncwarp();
         src += kSl / 2;
         if (++slot == kRing) {
           slot = 0;
@@ -578,8 +661,11 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
         }
       }
     }
-    flags[2] = (int)G;
-    if (!ok) flags[4] = 1;
+    if (leader) {
+      flags[2] = (int)G;
+      if (!ok) flags[4] = 1;
+    }
+    __syncwarp();
   } else if (warp >= 4 && warp < 4 + kEpiWarps) {
     // ---- epilogue: warp w reads TMEM lane quarter w % 4; with 8 warps the
     // two of a quarter take alternate 16-column groups
@@ -615,12 +701,18 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
       int b, zt, yt, xc;
       decode_tile(a, act, t, b, zt, yt, xc);
       const int acc = i & 1;
-      // one thread waits and tells the others, so that all of them leave
-      // together if the wait gives up (they meet at named barriers below)
-      if (et == 0) flags[5] = mbar_wait(&acc_full[acc], (uint32_t)(i >> 1) & 1u) ? 1 : 0;
-      epi_sync();
-      const bool ready = *reinterpret_cast<volatile int*>(&flags[5]) != 0;
-      epi_sync();
+      bool ready;
+      if (TF32) {
+        // tcgen05.ld is collective over a warp: its lanes leave together
+        ready = __all_sync(0xffffffffu, mbar_wait(&acc_full[acc], (uint32_t)(i >> 1) & 1u));
+      } else {
+        // one thread waits and tells the others, so that all of them leave
+        // together if the wait gives up (they meet at named barriers below)
+        if (et == 0) flags[5] = mbar_wait(&acc_full[acc], (uint32_t)(i >> 1) & 1u) ? 1 : 0;
+        epi_sync();
+        ready = *reinterpret_cast<volatile int*>(&flags[5]) != 0;
+        epi_sync();
+      }
       if (!ready) {
         ok = false;
         break;
@@ -840,11 +932,16 @@ void pack_taps(const float* h_filters, int nfilt, uint16_t* dst, bool tf32) {
 
 static int g_num_sms = 0;
 
-// Dynamic shared memory of a geometry: tap ring, two input buffers (hi and
-// lo, two K halves each), epilogue transpose buffer, barriers; at least
-// 116 KB, so that one CTA (and its 512 TMEM columns) is alone on its SM.
-static int smem_bytes(int NR) {
-  const int need = kRing * kSlotBytes + 128 * NR + kEpiBytes + kBarBytes;
+// Shared-memory offsets of a geometry: tap ring, two input buffers (hi and
+// lo, two K halves each), epilogue transpose buffer (BF16X3), barriers, the
+// staging's row table (at most NR rows).
+static int ring_bytes(bool tf32) { return kRing * (tf32 ? kSlotBytesSp : kSlotBytes); }
+static int bar_offset(int NR, bool tf32) { return ring_bytes(tf32) + 128 * NR + (tf32 ? 0 : kEpiBytes); }
+
+// Dynamic shared memory of a geometry; at least 116 KB, so that one CTA (and
+// its 512 TMEM columns) is alone on its SM.
+static int smem_bytes(int NR, bool tf32) {
+  const int need = bar_offset(NR, tf32) + kBarBytes + 8 * NR;
   return need > 116 * 1024 ? need : 116 * 1024;
 }
 
@@ -865,7 +962,7 @@ Geometry make_geometry(int nfilt, int H, int D, int Ty, bool tf32) {
   g.RP = ((qmax * g.Hp + 6 + g.N) + 7) / 8 * 8;
   g.NR = g.SP * g.RP;
   g.nstage = num_stages(nfilt);
-  g.smem = smem_bytes(g.NR);
+  g.smem = smem_bytes(g.NR, tf32);
   return g;
 }
 
@@ -954,9 +1051,10 @@ cudaError_t launch(const float* vol, int W, int H, int D, int batch, long long s
   if (ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
   a.tiles_per = a.nxc * a.nyt * a.nzt;
   a.nqp = (g.SP * g.J + 6) / g.SP;
-  a.in_off = (uint32_t)(kRing * kSlotBytes);
+  a.in_off = (uint32_t)ring_bytes(tf32);
   a.e_off = a.in_off + 128u * (uint32_t)g.NR;
-  a.bar_off = a.e_off + (uint32_t)kEpiBytes;
+  a.bar_off = (uint32_t)bar_offset(g.NR, tf32);
+  a.tab_off = a.bar_off + (uint32_t)kBarBytes;
   const int grid = ntiles < g_num_sms ? (int)ntiles : g_num_sms;
   if (tf32)
     filter3d_tc_kernel<true><<<grid, kThreads, g.smem, st>>>(vol, d_taps, out, a, g, act, d_err);
