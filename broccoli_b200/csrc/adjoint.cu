@@ -237,7 +237,8 @@ warp_affine_backward_kernel(const float* __restrict__ src, int W, int H, int D,
   for (int j = 0; j < 12; j++) acc[j] = 0.0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < V;
        i += (long long)gridDim.x * blockDim.x) {
-    const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+    int x, y, z;
+    voxel_of(i, W, H, x, y, z);
     const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
     const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
     const float zf = (float)z - ((float)D - 1.0f) * 0.5f;
@@ -304,7 +305,8 @@ warp_field_backward_kernel(const float* __restrict__ src, int W, int H, int D, c
   const long long V = (long long)W * H * D;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   float gx, gy, gz, wt[8];
   long long idx[8];
   sample_grad(src, W, H, D, (float)x + dx[i] + 0.5f, (float)y + dy[i] + 0.5f, (float)z + dz[i] + 0.5f, gx, gy,

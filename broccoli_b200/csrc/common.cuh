@@ -117,21 +117,64 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
   return r;
 }
 
+// Voxel i of a volume as (x, y, z): 32-bit divisions where the index allows
+// them (a 64-bit division by a runtime size is some hundred instructions,
+// more than the rest of an elementwise kernel).
+__device__ __forceinline__ void voxel_of(long long i, int W, int H, int& x, int& y, int& z) {
+  if ((i >> 32) == 0) {
+    const unsigned r = (unsigned)i / (unsigned)W;
+    x = (int)((unsigned)i - r * (unsigned)W);
+    z = (int)(r / (unsigned)H);
+    y = (int)(r - (unsigned)z * (unsigned)H);
+  } else {
+    x = (int)(i % W);
+    y = (int)((i / W) % H);
+    z = (int)(i / ((long long)W * H));
+  }
+}
+
+// floor(v) as a float and an integer, for |v| < 2^22: adding 1.5 x 2^23 with
+// rounding towards minus infinity leaves floor(v) in the low mantissa bits.
+// (floorf and the conversion to int are one operation each of the
+// quarter-rate unit; these are two additions and an integer subtraction.)
+__device__ __forceinline__ void floor_small(float v, float& f, int& i) {
+  const float t = __fadd_rd(v, 12582912.0f);
+  f = t - 12582912.0f;
+  i = __float_as_int(t) - 0x4B400000;
+}
+
 // OpenCL 1.2 section 8.2 linear filtering with unnormalised coordinates and
 // clamp-to-edge addressing, exact float weights (the sampler of
 // kernelRegistration.cpp:1064).  u, v, w include the +0.5 texel offset.
+//
+// A warp whose eight neighbours are all inside the volume takes one base
+// address and constant offsets; any other warp clamps every index, without a
+// branch per lane (at W = 64 every warp of a moved volume holds an edge, and
+// lanes that took two paths one after the other doubled its instructions).
 __device__ __forceinline__ float sample_linear(const float* __restrict__ T, int W, int H, int D,
                                               float u, float v, float w) {
   // volumes hold fewer than 2^31 voxels (checked by the launchers)
   const float uu = u - 0.5f, vv = v - 0.5f, ww = w - 0.5f;
-  const float fu = floorf(uu), fv = floorf(vv), fw = floorf(ww);
+  float fu, fv, fw;
+  int i0, j0, k0;
+  if (fmaxf(fmaxf(fabsf(uu), fabsf(vv)), fabsf(ww)) < 4194304.0f) {
+    floor_small(uu, fu, i0);
+    floor_small(vv, fv, j0);
+    floor_small(ww, fw, k0);
+  } else {
+    fu = floorf(uu);
+    fv = floorf(vv);
+    fw = floorf(ww);
+    i0 = (int)fu;
+    j0 = (int)fv;
+    k0 = (int)fw;
+  }
   const float a = uu - fu, bb = vv - fv, c = ww - fw;
-  const int i0 = (int)fu, j0 = (int)fv, k0 = (int)fw;
   const int WH = W * H;
   float t000, t100, t010, t110, t001, t101, t011, t111;
-  if ((unsigned)i0 < (unsigned)(W - 1) && (unsigned)j0 < (unsigned)(H - 1) && (unsigned)k0 < (unsigned)(D - 1)) {
-    // all eight neighbours inside the volume (the clamps below leave them
-    // as they are): one base address and constant offsets
+  const bool inside =
+      (unsigned)i0 < (unsigned)(W - 1) && (unsigned)j0 < (unsigned)(H - 1) && (unsigned)k0 < (unsigned)(D - 1);
+  if (__all_sync(__activemask(), inside)) {
     const float* p0 = T + (i0 + j0 * W + k0 * WH);
     const float* p1 = p0 + WH;
     t000 = __ldg(p0);
@@ -143,9 +186,10 @@ __device__ __forceinline__ float sample_linear(const float* __restrict__ T, int 
     t011 = __ldg(p1 + W);
     t111 = __ldg(p1 + W + 1);
   } else {
-    const int xi0 = min(max(i0, 0), W - 1), xi1 = min(max(i0 + 1, 0), W - 1);
-    const int yj0 = min(max(j0, 0), H - 1), yj1 = min(max(j0 + 1, 0), H - 1);
-    const int zk0 = min(max(k0, 0), D - 1), zk1 = min(max(k0 + 1, 0), D - 1);
+    // i0 + 1 of the largest int (a saturated conversion) clamps as i0 does
+    const int xi0 = min(max(i0, 0), W - 1), xi1 = min(max(i0, -1) + (i0 < W), W - 1);
+    const int yj0 = min(max(j0, 0), H - 1), yj1 = min(max(j0, -1) + (j0 < H), H - 1);
+    const int zk0 = min(max(k0, 0), D - 1), zk1 = min(max(k0, -1) + (k0 < D), D - 1);
     const int r00 = yj0 * W + zk0 * WH;
     const int r10 = yj1 * W + zk0 * WH;
     const int r01 = yj0 * W + zk1 * WH;

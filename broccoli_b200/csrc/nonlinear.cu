@@ -225,7 +225,8 @@ rescale_batch_kernel(const float* __restrict__ src, int W, int H, int D, float* 
   const long long V2 = (long long)W2 * H2 * D2;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
-  const int x = (int)(i % W2), y = (int)((i / W2) % H2), z = (int)(i / ((long long)W2 * H2));
+  int x, y, z;
+  voxel_of(i, W2, H2, x, y, z);
   const float v = sample_lin(src + (long long)b * W * H * D, W, H, D, x * vx + 0.5f, y * vy + 0.5f,
                              z * vz + 0.5f);
   out[(long long)b * V2 + i] = factor == 1.0f ? v : v * factor;
@@ -293,7 +294,8 @@ resize_to_grid_kernel(const float* __restrict__ src, int W, int H, int D, float*
   const long long V2 = (long long)W2 * H2 * D2;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
-  const int xn = (int)(i % W2), yn = (int)((i / W2) % H2), zn = (int)(i / ((long long)W2 * H2));
+  int xn, yn, zn;
+  voxel_of(i, W2, H2, xn, yn, zn);
   const int x = xn - g.offn[0], y = yn - g.offn[1], z = zn - g.offn[2];
   const int xi = x + g.offi[0], yi = y + g.offi[1], zi = z + g.offi[2];
   float v = 0.f;
@@ -317,7 +319,8 @@ resize_to_grid_ragged_kernel(const ResizeJob* __restrict__ jobs, float* __restri
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
   const ResizeJob& j = jobs[blockIdx.y];
-  const int xn = (int)(i % W2), yn = (int)((i / W2) % H2), zn = (int)(i / ((long long)W2 * H2));
+  int xn, yn, zn;
+  voxel_of(i, W2, H2, xn, yn, zn);
   const int x = xn - j.g.offn[0], y = yn - j.g.offn[1], z = zn - j.g.offn[2];
   const int xi = x + j.g.offi[0], yi = y + j.g.offi[1], zi = z + j.g.offi[2];
   float v = 0.f;
@@ -336,7 +339,8 @@ mass_moments_kernel(const float* __restrict__ vol, int W, int H, int D, double* 
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < V;
        i += (long long)gridDim.x * blockDim.x) {
     const double v = vol[i];
-    const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+    int x, y, z;
+    voxel_of(i, W, H, x, y, z);
     m += v;
     mx += v * x;
     my += v * y;
@@ -369,7 +373,8 @@ add_affine_to_field_kernel(float* __restrict__ field, int W, int H, int D, Param
   const long long V = (long long)W * H * D;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   const float* p = prm.p;
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
@@ -453,7 +458,8 @@ transform_affine_kernel(const float* __restrict__ src, int W, int H, int D, Para
   const long long V = (long long)W * H * D;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   const float* p = prm.p;
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
@@ -475,7 +481,8 @@ transform_field_kernel(const float* __restrict__ src, int W, int H, int D, const
   const long long V = (long long)W * H * D;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   const float u = __fadd_rn(__fadd_rn((float)x, __ldg(dx + i)), 0.5f);
   const float v = __fadd_rn(__fadd_rn((float)y, __ldg(dy + i)), 0.5f);
   const float w = __fadd_rn(__fadd_rn((float)z, __ldg(dz + i)), 0.5f);
@@ -491,7 +498,8 @@ combine_field_kernel(float* __restrict__ dx, float* __restrict__ dy, float* __re
   const long long V = (long long)W * H * D;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V) return;
-  const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   const float* p = prm.p;
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
@@ -513,7 +521,8 @@ resize_to_grid_mode_kernel(const float* __restrict__ src, int W, int H, int D, f
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
   const long long t = blockIdx.y;
-  const int xn = (int)(i % W2), yn = (int)((i / W2) % H2), zn = (int)(i / ((long long)W2 * H2));
+  int xn, yn, zn;
+  voxel_of(i, W2, H2, xn, yn, zn);
   const int x = xn - g.offn[0], y = yn - g.offn[1], z = zn - g.offn[2];
   const int xi = x + g.offi[0], yi = y + g.offi[1], zi = z + g.offi[2];
   float v = 0.f;

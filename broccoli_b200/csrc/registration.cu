@@ -882,8 +882,10 @@ warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, i
   const int x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y, z = blockIdx.y;
   if (x >= W || y >= H) return;
   const int n = active_count(act, batch);
+  const int* list = act.list ? act.list + (active_iteration(act) % 3) * act.stride : nullptr;
+  float* o = out + ((long long)z * H + y) * W + x;
   for (int li = blockIdx.z; li < n; li += gridDim.z) {
-    const int b = active_instance(act, li);
+    const int b = list ? __ldg(list + li) : li;
     float p[12];
     if (VEC) {
       const float4* p4 = reinterpret_cast<const float4*>(params + (long long)b * 12);
@@ -899,8 +901,7 @@ warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, i
 #pragma unroll
       for (int q = 0; q < 12; q++) p[q] = __ldg(params + (long long)b * 12 + q);
     }
-    out[(long long)b * out_stride + ((long long)z * H + y) * W + x] =
-        affine_sample(src + (long long)b * src_stride, W, H, D, p, x, y, z);
+    o[(long long)b * out_stride] = affine_sample(src + (long long)b * src_stride, W, H, D, p, x, y, z);
   }
 }
 
@@ -920,8 +921,8 @@ warp_field_kernel(const float* __restrict__ src, int W, int H, int D, const floa
   dy += b * field_stride;
   dz += b * field_stride;
   out += b * out_stride;
-  const int r = i / W;
-  const int x = i - r * W, y = r % H, z = r / H;
+  int x, y, z;
+  voxel_of(i, W, H, x, y, z);
   out[i] = sample_linear(src, W, H, D, (float)x + dx[i] + 0.5f, (float)y + dy[i] + 0.5f,
                          (float)z + dz[i] + 0.5f);
 }
@@ -934,8 +935,8 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
   const int V2 = W2 * H2 * D2;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
-  const int r = i / W2;
-  const int x = i - r * W2, y = r % H2, z = r / H2;
+  int x, y, z;
+  voxel_of(i, W2, H2, x, y, z);
   out[i] = sample_linear(src, W, H, D, x * vx + 0.5f, y * vy + 0.5f, z * vz + 0.5f);
 }
 
@@ -1343,7 +1344,8 @@ phase_volumes_kernel(const float2* __restrict__ q1, const float2* __restrict__ q
     }
   }
   if (grad) {
-    const int x = (int)(i % W), y = (int)((i / W) % H), z = (int)(i / ((long long)W * H));
+    int x, y, z;
+    voxel_of(i, W, H, x, y, z);
     const int c = axis == 0 ? x : (axis == 1 ? y : z);
     const int n = axis == 0 ? W : (axis == 1 ? H : D);
     const long long step = axis == 0 ? 1 : (axis == 1 ? (long long)W : (long long)W * H);
