@@ -56,7 +56,7 @@ static int nonlinear_step(brc_ctx* ctx, const float* q1, const float* q2, int G,
   BRC_TRY(ctx, brc::tensor_components(q2, V, m36, raw, st, G), "tensor_components");
   int s = ctx->smooth(raw, W, H, D, 6 * G, ft, ft, ft, nullptr, nullptr, ctx->tmp1.as<float>(), nullptr, t6, st);
   if (s != BRC_OK) return s;
-  BRC_TRY(ctx, brc::tensor_norm_max(t6, V, raw, maxbits, st, G, 6 * V, 9 * V), "tensor_norm_max");
+  BRC_TRY(ctx, brc::tensor_norm_max(t6, V, nullptr, maxbits, st, G, 6 * V), "tensor_norm_max");
   BRC_TRY(ctx, brc::nonlinear_ah(q1, q2, t6, V, maxbits, m36, dirs18, raw, raw + 6 * V, st, G, 9 * V),
           "nonlinear_ah");
   s = ctx->smooth(raw, W, H, D, 9 * G, fe, fe, fe, nullptr, nullptr, ctx->tmp1.as<float>(), nullptr, ah, st);

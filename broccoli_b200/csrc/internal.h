@@ -81,9 +81,10 @@ cudaError_t phase_volumes(const float* q1, const float* q2, int W, int H, int D,
 // dimension y): t6 / q2 hold 6 (complex) volumes per instance, a6 and h3
 // advance by ah_stride floats per instance, d3 by 3 volumes, maxbits by one
 // word; q1 (the reference's responses) is shared.
+// a11 (may be null): the norms.
 cudaError_t tensor_norm_max(const float* t6, long long V, float* a11, unsigned int* maxbits, cudaStream_t st,
                             int batch = 1, long long t_stride = 0, long long a_stride = 0);
-cudaError_t nonlinear_ah(const float* q1, const float* q2, float* t6, long long V,
+cudaError_t nonlinear_ah(const float* q1, const float* q2, const float* t6, long long V,
                          const unsigned int* maxbits, const float* m36, const float* dirs18, float* a6,
                          float* h3, cudaStream_t st, int batch = 1, long long ah_stride = 0);
 cudaError_t tensor_components(const float* q2, long long V, const float* m36, float* t6, cudaStream_t st,
