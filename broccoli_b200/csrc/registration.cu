@@ -228,7 +228,9 @@ normal_eq_partial_kernel(const float2* __restrict__ q1, long long q1_stride,
 
 constexpr int kMarchWarps = 10;              // 8 output rows + 2 halo rows
 constexpr int kMarchCols = 30;               // output columns per warp
+constexpr int kMarchThreads = kMarchWarps * 32;
 constexpr int kMarchZs = 32;                 // at most this many planes per slab (14: 3.5 % slower for a series)
+constexpr int kMarchMaxGs = 10;              // planes of a CTA of a shared slab (7.5 KB of shared memory each)
 
 constexpr int kMarchRowSums = 27;            // 9 row moments per axis (below)
 // Row moment of sum e (0..13) of an axis: [s0, x s0, xx s0, sz, x sz, szz, v0, x v0, vz].
@@ -247,11 +249,41 @@ __device__ __forceinline__ void load_plane_q(const float2* __restrict__ Q1, cons
   }
 }
 
-template <bool SMOOTH>
+// All threads of the CTAs of a cluster.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A float at the address `p` of this CTA's shared memory, read from CTA `rank`.
+__device__ __forceinline__ float cluster_load(const float* p, int rank) {
+  uint32_t a;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// Adds a plane's w and v to the moments of an axis.
+__device__ __forceinline__ void add_moments(float (&m)[5], float wv, float vv, float zf) {
+  m[0] += wv;
+  m[1] += wv * zf;
+  m[2] += wv * zf * zf;
+  m[3] += vv;
+  m[4] += vv * zf;
+}
+
+// SPLIT: a cluster of np CTAs shares a slab, gs planes each.  The CTAs keep the
+// w and v of their planes in shared memory and the first one adds them all
+// plane by plane, so that the FP32 moments are those of one CTA walking the
+// slab, bit for bit, and a volume's result does not depend on the batch it is
+// in.
+template <bool SMOOTH, bool SPLIT>
 __global__ void __launch_bounds__(kMarchWarps * 32, 2)
 normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const float2* __restrict__ q2, int W,
-                       int H, int D, int ntx, int nty, int zs, double* __restrict__ partials,
+                       int H, int D, int ntx, int nty, int zs, int gs, int np, double* __restrict__ partials,
                        const ActiveSet act, float cw0, float cw1) {
+  extern __shared__ float s_wv[];  // SPLIT: [gs planes][3 axes][w, v][threads]
   if ((int)blockIdx.y >= active_count(act, (int)gridDim.y)) return;
   const int b = active_instance(act, blockIdx.y);
   // Shared slots are numbered by step: the plane of step s (p = z0 - 1 + s)
@@ -266,14 +298,15 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
   const long long V = (long long)W * H * D;
   const long long WH = (long long)W * H;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nzs = gridDim.x / (ntx * nty);
-  const int zsl = blockIdx.x / (ntx * nty), rem = blockIdx.x - zsl * (ntx * nty);
+  const int part = SPLIT ? blockIdx.x % np : 0;
+  const int bx = SPLIT ? blockIdx.x / np : blockIdx.x, nbx = SPLIT ? gridDim.x / np : gridDim.x;
+  const int zsl = bx / (ntx * nty), rem = bx - zsl * (ntx * nty);
   const int yt = rem / ntx, xt = rem - yt * ntx;
   const int x = 3 + xt * kMarchCols - 1 + lane;  // lanes 0 and 31: halo columns
   const int y = 3 + yt * 8 - 1 + warp;           // warps 0 and 9: halo rows
-  const int z0 = 3 + zsl * zs;
-  const int z1 = min(D - 3, z0 + zs);
-  (void)nzs;
+  const int zend = min(D - 3, 3 + (zsl + 1) * zs);
+  const int z0 = 3 + zsl * zs + (SPLIT ? part * gs : 0);
+  const int z1 = SPLIT ? min(zend, z0 + gs) : zend;
   const bool empty = W <= 6 || H <= 6 || z1 <= z0;  // no interior voxel: zero sums
   const float2* Q1 = q1 + (long long)b * q1_stride;
   const float2* Q2 = q2 + (long long)b * 3 * V;
@@ -361,11 +394,13 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
           const float cg = cert * g;
           const float wv = cg * g;
           const float vv = cg * pd;
-          m[k][0] += wv;
-          m[k][1] += wv * zf;
-          m[k][2] += wv * zf * zf;
-          m[k][3] += vv;
-          m[k][4] += vv * zf;
+          if (SPLIT) {
+            float* t = s_wv + ((z - z0) * 6 + 2 * k) * kMarchThreads + threadIdx.x;
+            t[0] = wv;
+            t[kMarchThreads] = vv;
+          } else {
+            add_moments(m[k], wv, vv, zf);
+          }
         }
       }
     }
@@ -383,6 +418,27 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
     }
   }
 
+  if (SPLIT) {
+    cluster_sync();
+    if (part == 0 && out) {
+      for (int r = 0; r < np; r++) {
+        const int za = z0 + r * gs, zb = min(zend, za + gs);
+#pragma unroll 2
+        for (int z = za; z < zb; z++) {
+          const float zf = (float)z - 0.5f * (float)(D - 1);
+          const float* t = s_wv + (z - za) * (6 * kMarchThreads) + threadIdx.x;
+          float v[6];
+#pragma unroll
+          for (int q = 0; q < 6; q++) v[q] = cluster_load(t + q * kMarchThreads, r);
+#pragma unroll
+          for (int k = 0; k < 3; k++) add_moments(m[k], v[2 * k], v[2 * k + 1], zf);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync();  // no CTA leaves while its planes are read
+    if (part != 0) return;
+  }
   // FP64 sums over the row of a warp (y is the same for its lanes): nine
   // moments per axis, sum s0 [1, x, xx], sz [1, x], szz, v0 [1, x], vz.  The 27
   // sums over 32 lanes take one transposing tree of 31 exchanges (lane l ends
@@ -428,7 +484,7 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
       const double yd = (double)(3 + yt * 8 - 1 + w) - 0.5 * (double)(H - 1);
       v += s_part[w][q] * (py == 0 ? 1.0 : (py == 1 ? yd : yd * yd));
     }
-    partials[((long long)b * gridDim.x + blockIdx.x) * kNSums + threadIdx.x] = v;
+    partials[((long long)b * nbx + bx) * kNSums + threadIdx.x] = v;
   }
 }
 
@@ -1211,25 +1267,77 @@ int normal_eq_march_blocks(int W, int H, int D, int* ntx, int* nty, int* zs) {
   return *ntx * *nty * nzs;
 }
 
+// CTAs that share a slab: the most, up to a cluster's 8 and with six planes or more each,
+// that all run at once (two per SM); 1 where they would not.  Such a launch is a
+// chain of plane steps, which the parts shorten (one 64x64x33 volume: 16 CTAs of
+// 29 steps, or 80 of 8; 20 iterations 952 -> 827 us, with four planes each 835);
+// a larger one fills the chip with whole slabs, which step over two halo planes
+// once and not per part.
+static int march_parts(long long blocks, int zs) {
+  for (int np = 8; np > 1; np--) {
+    const int gs = (zs + np - 1) / np;
+    if (gs >= 6 && gs <= kMarchMaxGs && (np - 1) * gs < zs && blocks * np <= 2 * 148) return np;
+  }
+  return 1;
+}
+
+template <bool SMOOTH, bool SPLIT>
+static cudaError_t launch_march(const float2* q1, long long q1_stride, const float2* q2, int W, int H, int D, int ntx,
+                                int nty, int nblk, int zs, int np, int batch, double* partials, ActiveSet act,
+                                float w0, float w1, cudaStream_t st) {
+  const int gs = SPLIT ? (zs + np - 1) / np : zs;
+  const size_t plane = sizeof(float) * 6 * kMarchThreads;
+  if (SPLIT) {
+    // shared memory above 48 KB is a per-device function attribute
+    static bool attr_set[64] = {false};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!attr_set[dev]) {
+      const cudaError_t e = cudaFuncSetAttribute(normal_eq_march_kernel<SMOOTH, SPLIT>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)(plane * kMarchMaxGs));
+      if (e != cudaSuccess) return e;
+      attr_set[dev] = true;
+    }
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(nblk * np), (unsigned)batch);
+  cfg.blockDim = dim3(kMarchThreads);
+  cfg.dynamicSmemBytes = SPLIT ? plane * gs : 0;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)np;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = SPLIT ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, normal_eq_march_kernel<SMOOTH, SPLIT>, q1, q1_stride, q2, W, H, D, ntx, nty, zs, gs,
+                            np, partials, act, w0, w1);
+}
+
 cudaError_t normal_eq_march(const float* q1, long long q1_stride_floats, const float* q2, int W, int H, int D,
                             int batch, double* partials, int nblk, ActiveSet act, cudaStream_t st,
                             float cert_sigma) {
   int ntx, nty, zs;
   if (normal_eq_march_blocks(W, H, D, &ntx, &nty, &zs) != nblk) return cudaErrorInvalidValue;
-  dim3 grid((unsigned)nblk, (unsigned)batch);
   const float2* a = reinterpret_cast<const float2*>(q1);
   const float2* c = reinterpret_cast<const float2*>(q2);
+  const int np = march_parts((long long)nblk * batch, zs);
+  // 3-tap Gaussian of the certainties, weights normalised to sum 1
+  float w0 = 1.f, w1 = 0.f;
   if (cert_sigma > 0.f) {
-    // 3-tap Gaussian, weights normalised to sum 1
     const float e = (float)exp(-1.0 / (2.0 * (double)cert_sigma * (double)cert_sigma));
-    const float w0 = 1.0f / (1.0f + 2.0f * e), w1 = e * w0;
-    normal_eq_march_kernel<true><<<grid, kMarchWarps * 32, 0, st>>>(a, q1_stride_floats / 2, c, W, H, D, ntx, nty,
-                                                                     zs, partials, act, w0, w1);
-  } else {
-    normal_eq_march_kernel<false><<<grid, kMarchWarps * 32, 0, st>>>(a, q1_stride_floats / 2, c, W, H, D, ntx,
-                                                                      nty, zs, partials, act, 1.f, 0.f);
+    w0 = 1.0f / (1.0f + 2.0f * e);
+    w1 = e * w0;
   }
-  return cudaGetLastError();
+  const auto launch = [&](auto smooth, auto split) {
+    return launch_march<decltype(smooth)::value, decltype(split)::value>(
+        a, q1_stride_floats / 2, c, W, H, D, ntx, nty, nblk, zs, np, batch, partials, act, w0, w1, st);
+  };
+  if (cert_sigma > 0.f)
+    return np > 1 ? launch(std::true_type(), std::true_type()) : launch(std::true_type(), std::false_type());
+  return np > 1 ? launch(std::false_type(), std::true_type()) : launch(std::false_type(), std::false_type());
 }
 
 cudaError_t assemble_normal_eq(const double* partials, int nblk, int batch, double* A, double* h,

@@ -199,3 +199,21 @@ def test_certainty_smoothing_one_iteration_matches_oracle(ctx, orc, golden, lin_
     # and it differs from the unsmoothed solve
     r0 = ctx.register_linear(cuda(golden["base"]), cuda(golden["moved"])[None], lin_filters, 1, L.AFFINE)
     assert param_err(r0["params"].cpu().numpy()[0], p) > 10 * TOL
+
+
+@pytest.mark.parametrize("depth", [7, 15, 16, 33, 45])
+@pytest.mark.parametrize("sigma", [0.0, 1.0])
+def test_batch_size_does_not_change_a_registration(ctx, lin_filters, depth, sigma):
+    """A volume registered alone (its slabs split over clusters of CTAs) and
+    among 2,048 (one CTA per slab) gives the same parameters and aligned
+    volume bit for bit, at depths that leave one plane, one group, a group
+    and a remainder, and more than one slab inside the borders."""
+    rng = np.random.default_rng(depth)
+    ref = cuda(rng.standard_normal((depth, 12, 13)) * 100)
+    four = cuda(rng.standard_normal((4, depth, 12, 13)) * 100)
+    many = ctx.register_linear(ref, four.repeat(512, 1, 1, 1), lin_filters, 2, certainty_sigma=sigma)
+    for k in range(4):
+        one = ctx.register_linear(ref, four[k:k + 1], lin_filters, 2, certainty_sigma=sigma)
+        for name in ("params", "aligned"):
+            a, b = many[name][k::4], one[name]
+            assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b.expand_as(a)))
