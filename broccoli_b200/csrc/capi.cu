@@ -226,7 +226,7 @@ int brc_ctx::tune_fp32(const float* bank, brc::FilterKind kind, int nfilt, int W
   BRC_TRY(this, cudaStreamIsCapturing(stream(), &cap), "capture status");
   if (cap != cudaStreamCaptureStatusNone) return BRC_OK;  // no timing inside a capture
   int cand[8];
-  const int n = brc::filter3d_tz_candidates(cand, 8);
+  const int n = brc::filter3d_tz_candidates(nfilt, cand, 8);
   // time each z depth on zero-filled scratch volumes (the kernels' work does
   // not depend on the data, only on the shape and on whether the bank is
   // even/odd symmetric): one warm launch, best of three

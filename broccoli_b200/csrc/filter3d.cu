@@ -433,11 +433,19 @@ static cudaError_t set_smem_attr() {
 // context's tuner times them per volume shape (pick_tz is the untimed
 // choice).
 constexpr int kTzCandidates[] = {2, 3, 4, 6, 8};
+// kHalfRun + z depth: three filters with four outputs per thread in place of
+// eight, twice the warps for the same block.  A launch of one volume has a warp
+// or two per scheduler, which wait for their shared loads (one 64x64x33 volume:
+// 20 iterations of a registration 829 -> 769 us); a full chip prefers fewer
+// loads per FMA.
+constexpr int kHalfRun = 16;
 
 // Raises the dynamic shared-memory limit of every instantiation; called
 // once per device when a context is created.
 cudaError_t filter3d_init() {
   cudaError_t e;
+  if ((e = set_smem_attr<3, 4, 2>()) != cudaSuccess) return e;
+  if ((e = set_smem_attr<3, 4, 4>()) != cudaSuccess) return e;
 #define BRC_TZ_ATTR(TZ)                                                \
   if ((e = set_smem_attr<3, 8, TZ>()) != cudaSuccess) return e;        \
   if ((e = set_smem_attr<6, 4, TZ>()) != cudaSuccess) return e;
@@ -454,10 +462,14 @@ cudaError_t filter3d_init() {
 // exactly and 4 does not (e.g. D = 33), else 4.
 static int pick_tz(int D) { return (D % 4 != 0 && D % 3 == 0) ? 3 : 4; }
 
-int filter3d_tz_candidates(int* tz, int max_n) {
-  const int n = (int)(sizeof(kTzCandidates) / sizeof(kTzCandidates[0]));
-  for (int i = 0; i < n && i < max_n; i++) tz[i] = kTzCandidates[i];
-  return n < max_n ? n : max_n;
+int filter3d_tz_candidates(int nfilt, int* tz, int max_n) {
+  int n = 0;
+  for (int t : kTzCandidates)
+    if (n < max_n) tz[n++] = t;
+  if (nfilt == 3)
+    for (int t : {kHalfRun + 2, kHalfRun + 4})
+      if (n < max_n) tz[n++] = t;
+  return n;
 }
 
 int filter3d_default_tz(int D) { return pick_tz(D); }
@@ -489,17 +501,29 @@ cudaError_t filter3d_fp32(const float* vol, int W, int H, int D, int batch, long
                           FilterKind kind, int nfilt, float* out, ActiveSet act, cudaStream_t st, int tz) {
   if (tz <= 0) tz = pick_tz(D);
   if (nfilt != 3 && nfilt != 6) return cudaErrorInvalidValue;
+  const auto& sym3 = *reinterpret_cast<const SymBank<3>*>(bank);
+  const auto& all3 = *reinterpret_cast<const FilterBank<3>*>(bank);
+  if (nfilt == 3 && tz >= kHalfRun) {
+    switch (tz - kHalfRun) {
+      case 2:
+        return kind == kFilterSym ? launch_sym<3, 4, 2>(vol, W, H, D, batch, stride, sym3, out, act, st)
+                                  : launch_fp32<3, 4, 2>(vol, W, H, D, batch, stride, all3, out, act, st);
+      case 4:
+        return kind == kFilterSym ? launch_sym<3, 4, 4>(vol, W, H, D, batch, stride, sym3, out, act, st)
+                                  : launch_fp32<3, 4, 4>(vol, W, H, D, batch, stride, all3, out, act, st);
+      default: return cudaErrorInvalidValue;
+    }
+  }
   return dispatch_tz(tz, [&](auto T) {
     constexpr int kTz = decltype(T)::value;
+    if (nfilt == 3)
+      return kind == kFilterSym ? launch_sym<3, 8, kTz>(vol, W, H, D, batch, stride, sym3, out, act, st)
+                                : launch_fp32<3, 8, kTz>(vol, W, H, D, batch, stride, all3, out, act, st);
     if (kind == kFilterSym)
-      return nfilt == 3 ? launch_sym<3, 8, kTz>(vol, W, H, D, batch, stride,
-                                                *reinterpret_cast<const SymBank<3>*>(bank), out, act, st)
-                        : launch_sym<6, 4, kTz>(vol, W, H, D, batch, stride,
-                                                *reinterpret_cast<const SymBank<6>*>(bank), out, act, st);
-    return nfilt == 3 ? launch_fp32<3, 8, kTz>(vol, W, H, D, batch, stride,
-                                               *reinterpret_cast<const FilterBank<3>*>(bank), out, act, st)
-                      : launch_fp32<6, 4, kTz>(vol, W, H, D, batch, stride,
-                                               *reinterpret_cast<const FilterBank<6>*>(bank), out, act, st);
+      return launch_sym<6, 4, kTz>(vol, W, H, D, batch, stride, *reinterpret_cast<const SymBank<6>*>(bank), out, act,
+                                   st);
+    return launch_fp32<6, 4, kTz>(vol, W, H, D, batch, stride, *reinterpret_cast<const FilterBank<6>*>(bank), out, act,
+                                  st);
   });
 }
 

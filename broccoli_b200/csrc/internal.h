@@ -18,7 +18,7 @@ FilterKind filter3d_pack(const float* h_filters, int nfilt, bool allow_symmetric
 // untimed choice filter3d_default_tz(D).
 cudaError_t filter3d_fp32(const float* vol, int W, int H, int D, int batch, long long stride, const float* bank,
                           FilterKind kind, int nfilt, float* out, ActiveSet act, cudaStream_t st, int tz = 0);
-int filter3d_tz_candidates(int* tz, int max_n);
+int filter3d_tz_candidates(int nfilt, int* tz, int max_n);
 int filter3d_default_tz(int D);
 // registration.cu
 // Normal equations of batch instances, one CTA per `zpb` interior slices of
