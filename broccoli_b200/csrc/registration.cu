@@ -1007,7 +1007,7 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
 // passes (o = -4..4 in order, out-of-volume terms 0), and the volume is read
 // from HBM once and written once.
 //
-// A block owns a column tile of up to 64 x 8 outputs and marches along z
+// A block owns a column tile of up to 32 x 8 outputs and marches along z
 // through a chunk of planes, eight planes (a group) at a time:
 //   y  a thread takes one pair of window columns of a plane: sixteen 8-byte
 //      loads straight from global memory, 72 packed FMAs, eight 8-byte stores
@@ -1026,17 +1026,18 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
 // plane and a register ring for z issued 109 thread instructions per voxel
 // for its 27 FMAs.  Packed FP32 FMAs (two lanes per instruction, rounded as
 // two scalar ones) halve the issue slots of the arithmetic.
-// Measured (CUDA events): 9 volumes of 182x218x182 278 -> 174 us (3.0 TB/s),
-// 9 of 91x109x91 (odd width) 59 -> 37 us, 200 of 64x64x33 175 -> 73 us (3.0
+// Measured (CUDA events): 9 volumes of 182x218x182 278 -> 169 us (3.1 TB/s),
+// 9 of 91x109x91 (odd width) 59 -> 36 us, 200 of 64x64x33 175 -> 73 us (3.0
 // TB/s), the same with certainty, division and mask product in the kernel
-// 360 -> 173 us.  Issue is now 63 % and the FMA pipe 46 % of the cycles
-// (warps wait at the group's barriers and for the window's loads).
+// 360 -> 160 us.  Tiles of 64 columns with 288 threads: 174, 37, 73, 173 us
+// (fewer, larger blocks wait longer at a group's barriers); 48 columns 182, 40,
+// 83, 218.
 // `out` must not overlap the inputs.
-constexpr int kSmTX = 64, kSmTY = 8;    // largest output tile (the width is chosen per volume)
+constexpr int kSmTX = 32, kSmTY = 8;    // largest output tile (the width is chosen per volume)
 constexpr int kSmG = 8;                 // planes per group
-constexpr int kSmThreads = 288;         // y units of a 64-wide tile: 36 column pairs x 8 planes
-constexpr int kSmPY = kSmTX + 12;       // y buffer pitch: 76 floats, 12 modulo 32
-constexpr int kSmPR = kSmTX + 4;        // ring pitch: 68 floats, 4 modulo 32
+constexpr int kSmThreads = 160;         // y units of a 32-wide tile: 20 column pairs x 8 planes
+constexpr int kSmPY = kSmTX + 12;       // y buffer pitch: 44 floats, 12 modulo 32
+constexpr int kSmPR = kSmTX + 4;        // ring pitch: 36 floats, 4 modulo 32
 constexpr int kSmYPlane = kSmTY * kSmPY, kSmRPlane = kSmTY * kSmPR;
 constexpr int kSmRGroup = kSmG * kSmRPlane;
 constexpr size_t kSmSmem = sizeof(float) * (kSmG * kSmYPlane + 2 * kSmRGroup);
@@ -1048,7 +1049,7 @@ struct SmoothTaps {
   F2 x[9], y[9], z[9];
 };
 
-// Output width of a block's tile: W in equal parts of at most 64, rounded up to
+// Output width of a block's tile: W in equal parts of at most 32, rounded up to
 // whole octets of the x pass.
 __host__ __device__ inline int smooth_tile_width(int W) {
   const int n = (W + kSmTX - 1) / kSmTX;
@@ -1059,11 +1060,9 @@ __host__ __device__ inline int smooth_tile_width(int W) {
 // and 8-byte aligned volumes); DIV: divide by the smoothed certainty scert;
 // MUL: then multiply by the certainty; ACC: add into `out`.
 template <bool CERT, bool VEC, bool DIV, bool MUL, bool ACC>
-// Three blocks per SM (72 registers) where pairs move and there is no
-// certainty; the other forms spill there and run faster with two (odd width, 9
-// volumes of 91x109x91: 37 against 49 us; certainty, 200 volumes of 64x64x33:
-// 173 against 175 us).
-__global__ void __launch_bounds__(kSmThreads, VEC && !CERT ? 3 : 2)
+// Five blocks per SM where pairs move and there is no certainty; the other
+// forms spill there (certainty 194 against 160 us with four).
+__global__ void __launch_bounds__(kSmThreads, VEC && !CERT ? 5 : 4)
 smooth3d_kernel(const float* __restrict__ in, const float* __restrict__ cert, const float* __restrict__ scert,
                 int W, int H, int D, int tw, int zc, const __grid_constant__ SmoothTaps taps,
                 float* __restrict__ out) {

@@ -164,10 +164,11 @@ def test_smooth_normalized_matches_golden(ctx):
     assert np.abs(out[fin] - ref[fin]).max() <= TOL * np.abs(ref[fin]).max()
 
 
-@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 8, 2), (9, 9, 63), (8, 7, 64), (17, 8, 65), (16, 17, 128), (33, 5, 130)])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (7, 8, 2), (9, 9, 31), (8, 7, 32), (17, 8, 33), (9, 9, 63), (8, 7, 64), (17, 8, 65),
+                                   (16, 17, 128), (33, 5, 130)])
 @pytest.mark.parametrize("weighted", [False, True])
 def test_smoothing_tile_edges_vs_oracle(ctx, orc, shape, weighted):
-    """Sizes at the edges of the smoothing's 64 x 8 tiles, octets and groups
+    """Sizes at the edges of the smoothing's 32 x 8 tiles, octets and groups
     of eight planes, with odd and even widths (single and paired accesses),
     plain and as the normalised smoothing, whose quotient is multiplied by
     the mask in the same kernel.  Same bar as the golden tests, 1e-4."""
