@@ -200,8 +200,14 @@ tensor_components_kernel(const float2* __restrict__ q2, long long V, NonlinearCo
 // Linear resample of `batch` volumes to a new size, scaled by `factor`
 // (ChangeVolumeSize, broccoli_lib.cpp:6247-6388, followed by MultiplyVolume
 // for displacement fields, :6604-6611).
-__device__ __forceinline__ float sample_lin(const float* __restrict__ T, int W, int H, int D,
-                                            float u, float v, float w) {
+//
+// The eight clamped neighbours of a sample position and their weights: one
+// set serves the same position of several volumes.
+struct LinearTap {
+  long long o[8];
+  float w[8];
+};
+__device__ __forceinline__ void linear_tap(LinearTap& t, int W, int H, int D, float u, float v, float w) {
   const float uu = u - 0.5f, vv = v - 0.5f, ww = w - 0.5f;
   const float fu = floorf(uu), fv = floorf(vv), fw = floorf(ww);
   const float a = uu - fu, bb = vv - fv, c = ww - fw;
@@ -213,25 +219,59 @@ __device__ __forceinline__ float sample_lin(const float* __restrict__ T, int W, 
   const long long r10 = (long long)yj1 * W + (long long)zk0 * W * H;
   const long long r01 = (long long)yj0 * W + (long long)zk1 * W * H;
   const long long r11 = (long long)yj1 * W + (long long)zk1 * W * H;
-  return (1.f - a) * (1.f - bb) * (1.f - c) * __ldg(T + xi0 + r00) +
-         a * (1.f - bb) * (1.f - c) * __ldg(T + xi1 + r00) +
-         (1.f - a) * bb * (1.f - c) * __ldg(T + xi0 + r10) + a * bb * (1.f - c) * __ldg(T + xi1 + r10) +
-         (1.f - a) * (1.f - bb) * c * __ldg(T + xi0 + r01) + a * (1.f - bb) * c * __ldg(T + xi1 + r01) +
-         (1.f - a) * bb * c * __ldg(T + xi0 + r11) + a * bb * c * __ldg(T + xi1 + r11);
+  t.o[0] = xi0 + r00;
+  t.o[1] = xi1 + r00;
+  t.o[2] = xi0 + r10;
+  t.o[3] = xi1 + r10;
+  t.o[4] = xi0 + r01;
+  t.o[5] = xi1 + r01;
+  t.o[6] = xi0 + r11;
+  t.o[7] = xi1 + r11;
+  t.w[0] = (1.f - a) * (1.f - bb) * (1.f - c);
+  t.w[1] = a * (1.f - bb) * (1.f - c);
+  t.w[2] = (1.f - a) * bb * (1.f - c);
+  t.w[3] = a * bb * (1.f - c);
+  t.w[4] = (1.f - a) * (1.f - bb) * c;
+  t.w[5] = a * (1.f - bb) * c;
+  t.w[6] = (1.f - a) * bb * c;
+  t.w[7] = a * bb * c;
 }
+__device__ __forceinline__ float sample_tap(const float* __restrict__ T, const LinearTap& t) {
+  return t.w[0] * __ldg(T + t.o[0]) + t.w[1] * __ldg(T + t.o[1]) + t.w[2] * __ldg(T + t.o[2]) +
+         t.w[3] * __ldg(T + t.o[3]) + t.w[4] * __ldg(T + t.o[4]) + t.w[5] * __ldg(T + t.o[5]) +
+         t.w[6] * __ldg(T + t.o[6]) + t.w[7] * __ldg(T + t.o[7]);
+}
+__device__ __forceinline__ float sample_lin(const float* __restrict__ T, int W, int H, int D, float u, float v,
+                                            float w) {
+  LinearTap t;
+  linear_tap(t, W, H, D, u, v, w);
+  return sample_tap(T, t);
+}
+
+// Volumes a thread of rescale_batch_kernel takes one after the other: its
+// position and weights are most of the work (the fields of the pyramid;
+// T1-to-template, mixed precision: 12.84 -> 12.61 ms).
+constexpr int kRescaleVolumes = 3;
 
 __global__ void __launch_bounds__(256)
 rescale_batch_kernel(const float* __restrict__ src, int W, int H, int D, float* __restrict__ out, int W2,
-                     int H2, int D2, float vx, float vy, float vz, float factor) {
-  const int b = blockIdx.y;
+                     int H2, int D2, float vx, float vy, float vz, float factor, int batch) {
   const long long V2 = (long long)W2 * H2 * D2;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= V2) return;
   int x, y, z;
   voxel_of(i, W2, H2, x, y, z);
-  const float v = sample_lin(src + (long long)b * W * H * D, W, H, D, x * vx + 0.5f, y * vy + 0.5f,
-                             z * vz + 0.5f);
-  out[(long long)b * V2 + i] = factor == 1.0f ? v : v * factor;
+  LinearTap t;
+  linear_tap(t, W, H, D, x * vx + 0.5f, y * vy + 0.5f, z * vz + 0.5f);
+  const int b0 = blockIdx.y * kRescaleVolumes;
+#pragma unroll
+  for (int k = 0; k < kRescaleVolumes; k++) {
+    const int b = b0 + k;
+    if (b < batch) {
+      const float v = sample_tap(src + (long long)b * W * H * D, t);
+      out[(long long)b * V2 + i] = factor == 1.0f ? v : v * factor;
+    }
+  }
 }
 
 // Total = New * Old per instance with translations scaled by tscale (2 for
@@ -710,8 +750,8 @@ cudaError_t rescale_batch(const float* src, int W, int H, int D, int batch, floa
   const float vx = (float)(W - 1) / (float)(W2 - 1);
   const float vy = (float)(H - 1) / (float)(H2 - 1);
   const float vz = (float)(D - 1) / (float)(D2 - 1);
-  dim3 grid(grid1((long long)W2 * H2 * D2), batch);
-  rescale_batch_kernel<<<grid, 256, 0, st>>>(src, W, H, D, out, W2, H2, D2, vx, vy, vz, factor);
+  dim3 grid(grid1((long long)W2 * H2 * D2), (batch + kRescaleVolumes - 1) / kRescaleVolumes);
+  rescale_batch_kernel<<<grid, 256, 0, st>>>(src, W, H, D, out, W2, H2, D2, vx, vy, vz, factor, batch);
   return cudaGetLastError();
 }
 
