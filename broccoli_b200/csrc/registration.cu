@@ -776,7 +776,11 @@ __device__ double update_magnitude(const float* p, int W, int H, int D) {
 // act; instances whose update is not yet below tol go to list
 // (it + 1) % 3, and list (it + 2) % 3 (the one iteration it - 1 used) is
 // emptied for the next solve.
-__global__ void solve_update_kernel(const double* __restrict__ partials, int nblk, int type,
+//
+// Two blocks per SM: with the registers of one, the 199 instances of a series
+// took two rounds (25 us a launch, 16 now).
+__global__ void __launch_bounds__(kSolveThreads, 2)
+solve_update_kernel(const double* __restrict__ partials, int nblk, int type,
                                     float tol, int W, int H, int D, float* __restrict__ params,
                                     float* __restrict__ rotations, int* __restrict__ conv_iter,
                                     int* __restrict__ iterations, int* __restrict__ status,
