@@ -199,3 +199,30 @@ def test_filter_adjoint_tile_edges(shape, nf, offset, bank):
     assert fn(c.handle, AG._p(gd), W, H, D, 2, f.ctypes.data, nf, AG._p(out)) == 0
     err = (out.cpu().double() - ref).abs().max() / ref.abs().max()
     assert float(err) < 1e-4
+
+
+@pytest.mark.parametrize("shape", [(3, 5, 7), (6, 9, 8), (12, 16, 20)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_objective_equals_its_torch_form(shape, offset, lin_filters):
+    """The fused residual and sum of squares against the same objective from
+    the filtering and torch's elementwise operations: loss, gradient of the
+    parameters and of the reference responses, with reference responses that
+    are 16-byte aligned and that are not.  Both sum FP32 squares of the same
+    residuals in another order: 1e-5 relative."""
+    gen = torch.Generator().manual_seed(sum(shape))
+    moving = (torch.randn(shape, generator=gen) * 50 + 100).cuda()
+    q = AG.reference_responses((torch.randn(shape, generator=gen) * 50 + 100).cuda(), lin_filters, SIGMA)
+    buf = torch.empty(q.numel() + offset, device="cuda")
+    buf[offset:].copy_(q.reshape(-1))
+    grads = []
+    for fused in (True, False):
+        p = torch.tensor(_params(), dtype=torch.float32, device="cuda", requires_grad=True)
+        q_ref = buf[offset:].reshape(q.shape).detach().requires_grad_(True)
+        if fused:
+            loss = AG.registration_objective(moving, q_ref, lin_filters, SIGMA, params=p)
+        else:
+            w = AG.warp_affine(AG.smooth3d(moving[None], SIGMA), p.reshape(1, 12))
+            loss = ((AG.filter3d(w, lin_filters) - q_ref) ** 2).sum()
+        grads.append((loss.detach(),) + torch.autograd.grad(3.0 * loss, (p, q_ref)))
+    for a, b in zip(*grads):
+        assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
