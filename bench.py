@@ -714,8 +714,8 @@ def run_gpu(args, rank, world, local_rank):
     # is below the algorithmic bytes: the input comes partly from L2 (written
     # by the preceding resampling) and part of the output is still in L2
     # when the kernel ends.
-    tc_bytes_per_vol = ((34503168 + 148295936) if prec == L.PREC_TF32 else (17850368 + 48461056)) / 63
-    sym_bytes_per_vol = (34094848 + 147386624) / 63
+    tc_bytes_per_vol = ((34998528 + 148499968) if prec == L.PREC_TF32 else (34675456 + 148632064)) / 63
+    sym_bytes_per_vol = (34119936 + 144817664) / 63
     traffic = sym_bytes_per_vol * (T - 1) if symmetric_bank(fl) and tuple(SHAPE) == (33, 64, 64) else None
     tc_traffic = tc_bytes_per_vol * (T - 1) if tuple(SHAPE) == (33, 64, 64) else None
     achieved = f_flop / (f_ms / 1000.0) / 1e12
