@@ -117,6 +117,22 @@ __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
   return r;
 }
 
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_add_rm(F2 a, F2 b) {
+  F2 r;
+  asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) {
+  F2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // Voxel i of a volume as (x, y, z): 32-bit divisions where the index allows
 // them (a 64-bit division by a runtime size is some hundred instructions,
 // more than the rest of an elementwise kernel).
@@ -210,6 +226,74 @@ __device__ __forceinline__ float sample_linear(const float* __restrict__ T, int 
   return fmaf(c, c1 - c0, c0);
 }
 
+// The eight neighbours of (i0, j0, k0), every index clamped to the volume:
+// t[0] at (i0, j0, k0), + 1 for x, + 2 for y, + 4 for z.
+__device__ __forceinline__ void load_clamped(const float* __restrict__ T, int W, int H, int D, int i0, int j0,
+                                             int k0, float (&t)[8]) {
+  // clamped to [-1, W - 1] first: a saturated index then has a successor
+  const int ic = min(max(i0, -1), W - 1), jc = min(max(j0, -1), H - 1), kc = min(max(k0, -1), D - 1);
+  const int x0 = max(ic, 0), x1 = min(ic + 1, W - 1);
+  const int y0 = max(jc, 0), y1 = min(jc + 1, H - 1);
+  const int z0 = max(kc, 0) * H, z1 = min(kc + 1, D - 1) * H;
+  const int r00 = (y0 + z0) * W, r10 = (y1 + z0) * W, r01 = (y0 + z1) * W, r11 = (y1 + z1) * W;
+  t[0] = __ldg(T + (x0 + r00));
+  t[1] = __ldg(T + (x1 + r00));
+  t[2] = __ldg(T + (x0 + r10));
+  t[3] = __ldg(T + (x1 + r10));
+  t[4] = __ldg(T + (x0 + r01));
+  t[5] = __ldg(T + (x1 + r01));
+  t[6] = __ldg(T + (x0 + r11));
+  t[7] = __ldg(T + (x1 + r11));
+}
+
+// sample_linear at two positions at once (the halves of u, v, w), the
+// arithmetic as packed pairs: the same operations in the same order per half.
+__device__ __forceinline__ float2 sample_linear_pair(const float* __restrict__ T, int W, int H, int D, F2 u, F2 v,
+                                                     F2 w) {
+  const F2 half = f2_twice(0.5f), magic = f2_twice(12582912.0f);
+  const F2 uu = f2_sub(u, half), vv = f2_sub(v, half), ww = f2_sub(w, half);
+  const float2 us = f2_unpack(uu), vs = f2_unpack(vv), ws = f2_unpack(ww);
+  const float far = fmaxf(fmaxf(fmaxf(fabsf(us.x), fabsf(us.y)), fmaxf(fabsf(vs.x), fabsf(vs.y))),
+                          fmaxf(fabsf(ws.x), fabsf(ws.y)));
+  if (!(far < 4194304.0f)) {
+    const float2 u2 = f2_unpack(u), v2 = f2_unpack(v), w2 = f2_unpack(w);
+    return make_float2(sample_linear(T, W, H, D, u2.x, v2.x, w2.x), sample_linear(T, W, H, D, u2.y, v2.y, w2.y));
+  }
+  // floor_small of the six coordinates
+  const F2 tu = f2_add_rm(uu, magic), tv = f2_add_rm(vv, magic), tw = f2_add_rm(ww, magic);
+  const F2 a = f2_sub(uu, f2_sub(tu, magic)), b = f2_sub(vv, f2_sub(tv, magic)), c = f2_sub(ww, f2_sub(tw, magic));
+  const float2 iu = f2_unpack(tu), iv = f2_unpack(tv), iw = f2_unpack(tw);
+  const int ia = __float_as_int(iu.x) - 0x4B400000, ib = __float_as_int(iu.y) - 0x4B400000;
+  const int ja = __float_as_int(iv.x) - 0x4B400000, jb = __float_as_int(iv.y) - 0x4B400000;
+  const int ka = __float_as_int(iw.x) - 0x4B400000, kb = __float_as_int(iw.y) - 0x4B400000;
+  float ta[8], tb[8];
+  const bool inside = (unsigned)ia < (unsigned)(W - 1) && (unsigned)ja < (unsigned)(H - 1) &&
+                      (unsigned)ka < (unsigned)(D - 1) && (unsigned)ib < (unsigned)(W - 1) &&
+                      (unsigned)jb < (unsigned)(H - 1) && (unsigned)kb < (unsigned)(D - 1);
+  if (__all_sync(__activemask(), inside)) {
+    const long long WH = (long long)W * H;
+    const float* pa = T + (ia + (ja + ka * H) * W);
+    const float* pb = T + (ib + (jb + kb * H) * W);
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+      const long long o = ((q & 4) ? WH : 0) + ((q & 2) ? W : 0);
+      ta[q] = __ldg(pa + o + (q & 1));
+      tb[q] = __ldg(pb + o + (q & 1));
+    }
+  } else {
+    load_clamped(T, W, H, D, ia, ja, ka, ta);
+    load_clamped(T, W, H, D, ib, jb, kb, tb);
+  }
+  F2 t[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) t[q] = f2_pack(ta[q], tb[q]);
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) t[q] = f2_fma(a, f2_sub(t[q + 1], t[q]), t[q]);
+  t[0] = f2_fma(b, f2_sub(t[2], t[0]), t[0]);
+  t[4] = f2_fma(b, f2_sub(t[6], t[4]), t[4]);
+  return f2_unpack(f2_fma(c, f2_sub(t[4], t[0]), t[0]));
+}
+
 // The affine warp's sample of voxel (x, y, z): src at x + t + (A - I)(x -
 // centre) with p = {t, A - I} (InterpolateVolumeLinearLinear,
 // kernelRegistration.cpp:1066-1101).
@@ -222,6 +306,24 @@ __device__ __forceinline__ float affine_sample(const float* __restrict__ src, in
   const float v = (float)y + p[1] + p[6] * xf + p[7] * yf + p[8] * zf + 0.5f;
   const float w = (float)z + p[2] + p[9] * xf + p[10] * yf + p[11] * zf + 0.5f;
   return sample_linear(src, W, H, D, u, v, w);
+}
+
+// affine_sample of voxels (x, y, z) and (x, y, z2), the same bits.
+__device__ __forceinline__ float2 affine_sample_pair(const float* __restrict__ src, int W, int H, int D,
+                                                     const float* __restrict__ p, int x, int y, int z, int z2) {
+  const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
+  const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
+  const F2 zz = f2_pack((float)z, (float)z2);
+  const F2 zf = f2_sub(zz, f2_twice(((float)D - 1.0f) * 0.5f));
+  const F2 half = f2_twice(0.5f);
+  const float pu = fmaf(p[4], yf, fmaf(p[3], xf, (float)x + p[0]));
+  const float pv = fmaf(p[7], yf, fmaf(p[6], xf, (float)y + p[1]));
+  const F2 pw = f2_fma(f2_pack(p[10], p[10]), f2_pack(yf, yf),
+                       f2_fma(f2_pack(p[9], p[9]), f2_pack(xf, xf), f2_add(zz, f2_pack(p[2], p[2]))));
+  const F2 u = f2_add(f2_fma(f2_pack(p[5], p[5]), zf, f2_pack(pu, pu)), half);
+  const F2 v = f2_add(f2_fma(f2_pack(p[8], p[8]), zf, f2_pack(pv, pv)), half);
+  const F2 w = f2_add(f2_fma(f2_pack(p[11], p[11]), zf, pw), half);
+  return sample_linear_pair(src, W, H, D, u, v, w);
 }
 
 }  // namespace brc

@@ -931,19 +931,31 @@ __global__ void solve_given_kernel(const double* __restrict__ A, const double* _
 // (InterpolateVolumeLinearLinear, kernelRegistration.cpp:1066-1101).
 // VEC: params is 16-byte aligned, and the 12 parameters of an instance are
 // read as three 16-byte loads.
-template <bool VEC>
+//
+// Bound by instruction issue (one voxel per thread: 84 % of the slots at 178
+// instructions per warp and voxel row, 60 of them the list, parameters and
+// pointers of the instance; LSU 44 %, DRAM 8 %).  A thread takes the same
+// voxel of two planes: the instance's part and the x and y terms once, the
+// positions and interpolations as packed pairs.  One plane to two, us:
+// 199 x 64x64x33 135.0 -> 123.8-125.2, 59 x 80x80x37 88.3 -> 78.1, 24 x 64x64x33
+// 22.9 -> 19.1, one 182x218x182 53.5 -> 39.2.  56 registers, four blocks per SM; five and six blocks are slower
+// (130.6 and 139.5 us at the first size), as is clamping x alone where y and z
+// are inside (121.8 us there, but 43.3 at 182x218x182).
+template <bool VEC, int NZ>
 __global__ void __launch_bounds__(256)
 warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, int H, int D, int ntx, int batch,
                    const float* __restrict__ params, float* __restrict__ out, long long out_stride,
                    const ActiveSet act) {
-  // block: 32 x 8 voxels of one plane; grid (x-y tiles, planes, a share of
-  // the instances: blockIdx.z, + gridDim.z, ...)
+  // block: 32 x 8 voxels of NZ planes, a voxel of each per thread; grid (x-y
+  // tiles, groups of planes, a share of the instances: blockIdx.z, + gridDim.z, ...)
   const int ty = blockIdx.x / ntx, tx = blockIdx.x - ty * ntx;
-  const int x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y, z = blockIdx.y;
+  const int x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y, z = NZ * blockIdx.y;
   if (x >= W || y >= H) return;
+  const int z2 = min(z + 1, D - 1);
+  const long long WH = (long long)W * H;
   const int n = active_count(act, batch);
   const int* list = act.list ? act.list + (active_iteration(act) % 3) * act.stride : nullptr;
-  float* o = out + ((long long)z * H + y) * W + x;
+  float* o = out + z * WH + (y * W + x);
   for (int li = blockIdx.z; li < n; li += gridDim.z) {
     const int b = list ? __ldg(list + li) : li;
     float p[12];
@@ -961,7 +973,15 @@ warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, i
 #pragma unroll
       for (int q = 0; q < 12; q++) p[q] = __ldg(params + (long long)b * 12 + q);
     }
-    o[(long long)b * out_stride] = affine_sample(src + (long long)b * src_stride, W, H, D, p, x, y, z);
+    const float* s = src + (long long)b * src_stride;
+    float* ob = o + (long long)b * out_stride;
+    if constexpr (NZ == 2) {
+      const float2 r = affine_sample_pair(s, W, H, D, p, x, y, z, z2);
+      ob[0] = r.x;
+      if (z + 1 < D) ob[WH] = r.y;
+    } else {
+      ob[0] = affine_sample(s, W, H, D, p, x, y, z);
+    }
   }
 }
 
@@ -1383,13 +1403,17 @@ cudaError_t warp_affine(const float* src, long long src_stride, int W, int H, in
   const int ntx = (W + 31) / 32, nty = (H + 7) / 8;
   // at most 16 instance shares: a launch whose instances have mostly
   // converged does not pay for blocks with nothing to do
-  dim3 grid((unsigned)(ntx * nty), (unsigned)D, (unsigned)(batch < 16 ? batch : 16));
-  if ((reinterpret_cast<uintptr_t>(params) & 15) == 0)
-    warp_affine_kernel<true><<<grid, dim3(32, 8), 0, st>>>(src, src_stride, W, H, D, ntx, batch, params, out,
-                                                         out_stride, act);
-  else
-    warp_affine_kernel<false><<<grid, dim3(32, 8), 0, st>>>(src, src_stride, W, H, D, ntx, batch, params, out,
-                                                          out_stride, act);
+  const int shares = batch < 16 ? batch : 16;
+  // Two planes per thread where their blocks fill the chip (four per SM are
+  // resident); a smaller launch is as long as its busiest SM's chain, and half
+  // the blocks are spread less evenly (one 64x64x33: a registration of 20 such
+  // launches 767 us with two planes per thread, 762 with one).
+  const bool two = (long long)ntx * nty * ((D + 1) / 2) * shares >= 4 * 148;
+  const bool vec = (reinterpret_cast<uintptr_t>(params) & 15) == 0;
+  dim3 grid((unsigned)(ntx * nty), (unsigned)(two ? (D + 1) / 2 : D), (unsigned)shares);
+  auto* k = two ? (vec ? warp_affine_kernel<true, 2> : warp_affine_kernel<false, 2>)
+                : (vec ? warp_affine_kernel<true, 1> : warp_affine_kernel<false, 1>);
+  k<<<grid, dim3(32, 8), 0, st>>>(src, src_stride, W, H, D, ntx, batch, params, out, out_stride, act);
   return cudaGetLastError();
 }
 

@@ -104,6 +104,44 @@ def test_warp_affine_matches_golden(ctx, golden):
     assert rel_err(out.cpu().numpy()[0], golden["warp_affine"]) < TOL
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 7, 9), (2, 8, 32), (3, 33, 31), (5, 1, 1), (33, 64, 64), (6, 9, 65),
+                                   (148, 8, 63), (49, 50, 70), (3, 97, 165), (1, 120, 300)])
+def test_warp_affine_pairs_of_planes(ctx, shape):
+    """Odd and single planes, ragged tiles, positions on every side of the
+    volume, and positions no 32-bit index holds, against the clamped trilinear
+    sample in FP64."""
+    D, H, W = shape
+    g = torch.Generator().manual_seed(7)
+    vol = torch.randn((4, D, H, W), generator=g)
+    p = torch.randn((4, 12), generator=g) * 0.02
+    p[:, :3] *= 100.0
+    p[2, :3] = torch.tensor([1e7, -1e7, 0.25])
+    p[3, :3] = torch.tensor([-0.5, 3e9, -3e9])
+    out = ctx.warp_affine(vol.cuda(), p.cuda()).cpu().double()
+    z, y, x = torch.meshgrid(*[torch.arange(n, dtype=torch.float64) for n in shape], indexing="ij")
+    rel = [c - (n - 1) / 2 for c, n in ((x, W), (y, H), (z, D))]
+    for b in range(4):
+        q = p[b].double()
+        lo, hi, fr = [], [], []
+        for k, (c, n) in enumerate(((x, W), (y, H), (z, D))):
+            pos = c + q[k] + sum(q[3 + 3 * k + j] * rel[j] for j in range(3))
+            f = pos.floor()
+            lo.append(f.clamp(0, n - 1).long())
+            hi.append((f + 1).clamp(0, n - 1).long())
+            fr.append(pos - f)
+        ref = torch.zeros(shape, dtype=torch.float64)
+        for corner in range(8):
+            i = [hi[k] if corner >> k & 1 else lo[k] for k in range(3)]
+            w = [fr[k] if corner >> k & 1 else 1 - fr[k] for k in range(3)]
+            ref += w[0] * w[1] * w[2] * vol[b].double()[i[2], i[1], i[0]]
+        # a position takes six roundings of at most half a step of its
+        # magnitude (below 128: 2^-18); the sample's slope along an axis is at
+        # most twice the largest value
+        half = 2.0 ** (np.ceil(np.log2(1.2 * max(shape) + 16)) - 25)
+        tol = (3 * 2 * 6 * half + 8 * 2.0**-23) * float(vol.abs().max())
+        assert (out[b] - ref).abs().max() <= tol
+
+
 def test_warp_field_matches_golden(ctx, golden):
     out = ctx.warp_field(cuda(golden["moved"]), cuda(golden["field_x"]), cuda(golden["field_y"]),
                          cuda(golden["field_z"]))
