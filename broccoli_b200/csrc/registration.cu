@@ -933,8 +933,7 @@ __global__ void solve_given_kernel(const double* __restrict__ A, const double* _
 // read as three 16-byte loads.
 //
 // Bound by instruction issue (one voxel per thread: 84 % of the slots at 178
-// instructions per warp and voxel row, 60 of them the list, parameters and
-// pointers of the instance; LSU 44 %, DRAM 8 %).  A thread takes the same
+// instructions per warp and voxel row; LSU 44 %, DRAM 8 %).  A thread takes the same
 // voxel of two planes: the instance's part and the x and y terms once, the
 // positions and interpolations as packed pairs.  One plane to two, us:
 // 199 x 64x64x33 135.0 -> 123.8-125.2, 59 x 80x80x37 88.3 -> 78.1, 24 x 64x64x33
