@@ -39,14 +39,14 @@ def _ctx(device: torch.device) -> Context:
     return c
 
 
-def _sig(name, args):
+_P, _I, _Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
+
+
+def _sig(name, args, res=_I):
     fn = getattr(L.lib(), name)
     fn.argtypes = args
-    fn.restype = ctypes.c_int
+    fn.restype = res
     return fn
-
-
-_P, _I = ctypes.c_void_p, ctypes.c_int
 
 
 def gaussian_taps(sigma: float) -> np.ndarray:
@@ -152,9 +152,13 @@ class FilterSsd(torch.autograd.Function):
         r = q_ref.detach().contiguous()
         res = torch.empty_like(r)
         loss = torch.empty((), dtype=torch.float32, device=v.device)
-        fn = _sig("brc_filter3d_ssd", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P])
+        # the context is shared by all streams of the device: the block sums
+        # are torch's memory, like the residual
+        size = _sig("brc_filter3d_ssd_scratch_bytes", [_I] * 5, _Z)(W, H, D, B, f.shape[0])
+        sums = torch.empty(size, dtype=torch.uint8, device=v.device)
+        fn = _sig("brc_filter3d_ssd_scratch", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _Z])
         _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), f.shape[0], _p(r), _p(res),
-                     _p(loss)))
+                     _p(loss), _p(sums), size))
         fctx.filters = f
         fctx.save_for_backward(res)
         return loss

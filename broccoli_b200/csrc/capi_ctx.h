@@ -82,6 +82,7 @@ struct brc_ctx {
   // loops stop on the device, so their kernel count is known only there)
   DevBuf iters_run;
   DevBuf smask;   // smoothed certainty of brc_smooth_normalized
+  DevBuf ssd_sums;  // block sums of brc_filter3d_ssd (one size, allocated once)
   // tensor-core tile height chosen by timing, per (nfilt, W, H, D)
   std::map<std::tuple<int, int, int, int>, int> tc_tuned;
   // (nfilt + 100 sym, W, H, D, volumes timed) -> z depth
@@ -148,7 +149,7 @@ struct brc_ctx {
     return q1.bytes + q2.bytes + aligned.bytes + partials.bytes + ctl.bytes + tmp1.bytes +
            tmp2.bytes + series.bytes + corrected.bytes + params.bytes + rot.bytes + nl.bytes + pyr.bytes +
            r2v_work.bytes + r2v_lin.bytes + r2v_prm.bytes + coh_res.bytes + coh_mat.bytes + coh_lin.bytes +
-           coh_prm.bytes + coh_jobs.bytes;
+           coh_prm.bytes + coh_jobs.bytes + ssd_sums.bytes;
   }
 };
 

@@ -812,20 +812,40 @@ extern "C" int brc_filter3d_adjoint(brc_ctx* ctx, const float* d_grad, int W, in
   return BRC_OK;
 }
 
+extern "C" size_t brc_filter3d_ssd_scratch_bytes(int W, int H, int D, int batch, int nfilt) {
+  if (W <= 0 || H <= 0 || D <= 0 || batch <= 0 || (nfilt != 3 && nfilt != 6)) return 0;
+  return sizeof(double) * (size_t)brc::ssd_blocks(2ll * nfilt * W * H * D * batch);
+}
+
+extern "C" int brc_filter3d_ssd_scratch(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch,
+                                        const float* h_filters, int nfilt, const float* d_ref, float* d_residual,
+                                        float* d_loss, void* d_scratch, size_t scratch_bytes) {
+  if (!ctx) return BRC_ERR_INVALID;
+  if (!d_ref || !d_residual || !d_loss || d_ref == d_residual || !d_scratch ||
+      (reinterpret_cast<uintptr_t>(d_scratch) & 7) != 0 ||
+      scratch_bytes < brc_filter3d_ssd_scratch_bytes(W, H, D, batch, nfilt))
+    return ctx->fail(BRC_ERR_INVALID, "brc_filter3d_ssd: bad argument");
+  const int s = brc_filter3d(ctx, d_vol, W, H, D, batch, (long long)W * H * D, h_filters, nfilt, BRC_PREC_FP32,
+                             d_residual);
+  if (s != BRC_OK) return s;
+  const long long n = 2ll * nfilt * W * H * D * batch;
+  BRC_TRY(ctx, brc::ssd_residual(d_residual, d_ref, n, static_cast<double*>(d_scratch), d_loss, ctx->stream()), "ssd");
+  ctx->launches += 2;
+  return BRC_OK;
+}
+
+// The block sums in the context: a buffer of the largest size, which never
+// moves, so that a captured call stays valid for the context's life.
 extern "C" int brc_filter3d_ssd(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch,
                                 const float* h_filters, int nfilt, const float* d_ref, float* d_residual,
                                 float* d_loss) {
   if (!ctx) return BRC_ERR_INVALID;
   if (!d_ref || !d_residual || !d_loss || d_ref == d_residual)
     return ctx->fail(BRC_ERR_INVALID, "brc_filter3d_ssd: bad argument");
-  const int s = brc_filter3d(ctx, d_vol, W, H, D, batch, (long long)W * H * D, h_filters, nfilt, BRC_PREC_FP32,
-                             d_residual);
-  if (s != BRC_OK) return s;
-  const long long n = 2ll * nfilt * W * H * D * batch;
-  BRC_TRY(ctx, ctx->partials.ensure(sizeof(double) * (size_t)brc::ssd_blocks(n)), "alloc");
-  BRC_TRY(ctx, brc::ssd_residual(d_residual, d_ref, n, ctx->partials.as<double>(), d_loss, ctx->stream()), "ssd");
-  ctx->launches += 2;
-  return BRC_OK;
+  cudaSetDevice(ctx->device);
+  BRC_TRY(ctx, ctx->ssd_sums.ensure(sizeof(double) * (size_t)brc::ssd_blocks(1ll << 62)), "alloc");
+  return brc_filter3d_ssd_scratch(ctx, d_vol, W, H, D, batch, h_filters, nfilt, d_ref, d_residual, d_loss,
+                                  ctx->ssd_sums.ptr, ctx->ssd_sums.bytes);
 }
 
 extern "C" int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, int W, int H, int D, int batch,

@@ -309,9 +309,21 @@ int brc_filter3d_adjoint(brc_ctx* ctx, const float* d_grad, int W, int H, int D,
  * (the same layout) into d_residual, and the sum of the squares into d_loss
  * (one float).  brc_filter3d_ssd_adjoint is its adjoint: d_out = dL/dvol =
  * 2 *d_grad_loss times the adjoint filtering of the residual (d_grad_loss one
- * device float, dL/dloss).  No counterpart in the reference. */
+ * device float, dL/dloss).  No counterpart in the reference.
+ *
+ * The sum goes through the block sums of the residual kernel.
+ * brc_filter3d_ssd keeps them in the context (a fixed buffer), so its calls
+ * on one context must follow one another on the GPU;
+ * brc_filter3d_ssd_scratch keeps them in d_scratch, which the caller
+ * allocates for this call (8-byte aligned, at least
+ * brc_filter3d_ssd_scratch_bytes; else BRC_ERR_INVALID), so that calls on
+ * several streams, or captured in graphs, share nothing. */
 int brc_filter3d_ssd(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch, const float* h_filters,
                      int nfilt, const float* d_ref, float* d_residual, float* d_loss);
+size_t brc_filter3d_ssd_scratch_bytes(int W, int H, int D, int batch, int nfilt);
+int brc_filter3d_ssd_scratch(brc_ctx* ctx, const float* d_vol, int W, int H, int D, int batch,
+                             const float* h_filters, int nfilt, const float* d_ref, float* d_residual,
+                             float* d_loss, void* d_scratch, size_t scratch_bytes);
 int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, int W, int H, int D, int batch,
                              const float* h_filters, int nfilt, const float* d_grad_loss, float* d_out);
 

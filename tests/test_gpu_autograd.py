@@ -226,3 +226,74 @@ def test_objective_equals_its_torch_form(shape, offset, lin_filters):
         grads.append((loss.detach(),) + torch.autograd.grad(3.0 * loss, (p, q_ref)))
     for a, b in zip(*grads):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
+
+
+def _objective_inputs(shape, seed, lin_filters):
+    gen = torch.Generator().manual_seed(seed)
+    moving = (torch.randn(shape, generator=gen) * 50 + 100).cuda()
+    q = AG.reference_responses((torch.randn(shape, generator=gen) * 50 + 100).cuda(), lin_filters, SIGMA)
+    field = (torch.rand((3,) + tuple(shape), generator=gen) - 0.5).cuda()
+    return moving, q, field
+
+
+def test_objective_keeps_no_sums_in_the_shared_context(lin_filters, monkeypatch):
+    """One context serves every stream of a device, so the objective may hold
+    no per-call sums in it: a field objective after a filtering and a
+    smoothing of the same volume leaves the context's workspace as it was."""
+    monkeypatch.setattr(AG, "_contexts", {})
+    moving, q, field = _objective_inputs((9, 12, 10), 5, lin_filters)
+    before = AG._ctx(moving.device).workspace_bytes
+    AG.registration_objective(moving, q, lin_filters, SIGMA, field=field)
+    assert AG._ctx(moving.device).workspace_bytes == before
+
+
+def test_objectives_on_two_streams(lin_filters):
+    """Objectives queued alternately on two streams, the large and the small
+    one of each round free to run at once, give the losses of calls that run
+    alone, bit for bit (a fixed order of sums)."""
+    cases = [_objective_inputs(s, i, lin_filters) for i, s in enumerate([(40, 64, 64), (12, 20, 16)])]
+    alone = []
+    for m, q, f in cases:
+        alone.append(AG.registration_objective(m, q, lin_filters, SIGMA, field=f))
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    for s in streams:
+        s.wait_stream(torch.cuda.current_stream())
+    losses = []
+    for _ in range(20):
+        for (m, q, f), s in zip(cases, streams):
+            with torch.cuda.stream(s):
+                losses.append(AG.registration_objective(m, q, lin_filters, SIGMA, field=f))
+    torch.cuda.synchronize()
+    for k, loss in enumerate(losses):
+        assert torch.equal(loss, alone[k % 2])
+
+
+def test_captured_objective_outlives_later_calls(lin_filters, monkeypatch):
+    """A field objective captured in a CUDA graph replays to the eager loss
+    and gradient after calls that make the context grow: it holds no memory
+    of the context."""
+    monkeypatch.setattr(AG, "_contexts", {})
+    m, q, f = _objective_inputs((10, 14, 12), 3, lin_filters)
+    f.requires_grad_(True)
+
+    def step():
+        loss = AG.registration_objective(m, q, lin_filters, SIGMA, field=f)
+        return (loss.detach(),) + torch.autograd.grad(loss, f)
+
+    eager = step()
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step()
+    torch.cuda.current_stream().wait_stream(stream)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = step()
+    m2, q2, _ = _objective_inputs((40, 64, 64), 4, lin_filters)
+    p = torch.tensor(_params(), dtype=torch.float32, device="cuda", requires_grad=True)
+    AG.registration_objective(m2, q2, lin_filters, SIGMA, params=p).backward()
+    g.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(captured, eager):
+        assert torch.equal(a, b)
