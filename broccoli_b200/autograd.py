@@ -27,6 +27,8 @@ import torch
 from . import _lib as L
 from .api import Context, _check, _host_filters, _p
 
+# One context per device, shared by all its streams: an operation that needs
+# memory during its call takes torch's, on its own stream.
 _contexts = {}
 
 
@@ -90,8 +92,11 @@ class WarpAffine(torch.autograd.Function):
         B, D, H, W = (s.shape if s.dim() == 4 else (1,) + tuple(s.shape))
         gp = torch.empty((B, 12), dtype=torch.float64, device=g.device)
         gs = torch.empty((B, D, H, W), dtype=torch.float32, device=g.device) if fctx.needs_input_grad[0] else None
-        fn = _sig("brc_warp_affine_backward", [_P, _P, _I, _I, _I, _I, _P, _P, _P, _P])
-        _check(c, fn(c.handle, _p(s), W, H, D, B, _p(p), _p(g.contiguous()), _p(gp), _p(gs) if gs is not None else None))
+        size = _sig("brc_warp_affine_backward_scratch_bytes", [_I] * 4, _Z)(W, H, D, B)
+        sums = torch.empty(size, dtype=torch.uint8, device=g.device)
+        fn = _sig("brc_warp_affine_backward_scratch", [_P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _Z])
+        _check(c, fn(c.handle, _p(s), W, H, D, B, _p(p), _p(g.contiguous()), _p(gp),
+                     _p(gs) if gs is not None else None, _p(sums), size))
         gsrc = gs.reshape(s.shape) if gs is not None else None
         return gsrc, gp.to(torch.float32).reshape(fctx.saved_tensors[1].shape)
 
@@ -152,8 +157,7 @@ class FilterSsd(torch.autograd.Function):
         r = q_ref.detach().contiguous()
         res = torch.empty_like(r)
         loss = torch.empty((), dtype=torch.float32, device=v.device)
-        # the context is shared by all streams of the device: the block sums
-        # are torch's memory, like the residual
+        # the block sums are torch's memory (as the rows of WarpAffine.backward)
         size = _sig("brc_filter3d_ssd_scratch_bytes", [_I] * 5, _Z)(W, H, D, B, f.shape[0])
         sums = torch.empty(size, dtype=torch.uint8, device=v.device)
         fn = _sig("brc_filter3d_ssd_scratch", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _Z])

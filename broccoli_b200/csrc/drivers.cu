@@ -861,6 +861,11 @@ extern "C" int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, i
   return BRC_OK;
 }
 
+extern "C" size_t brc_warp_affine_backward_scratch_bytes(int W, int H, int D, int batch) {
+  if (W <= 0 || H <= 0 || D <= 0 || batch <= 0) return 0;
+  return sizeof(double) * 12 * (size_t)brc::warp_affine_backward_blocks((long long)W * H * D) * (size_t)batch;
+}
+
 extern "C" int brc_warp_affine_backward(brc_ctx* ctx, const float* d_src, int W, int H, int D, int batch,
                                         const float* d_params, const float* d_grad_out, double* d_grad_params,
                                         float* d_grad_src) {
@@ -869,13 +874,27 @@ extern "C" int brc_warp_affine_backward(brc_ctx* ctx, const float* d_src, int W,
       batch > 65535)
     return ctx->fail(BRC_ERR_INVALID, "brc_warp_affine_backward: bad argument");
   cudaSetDevice(ctx->device);
+  BRC_TRY(ctx, ctx->partials.ensure(brc_warp_affine_backward_scratch_bytes(W, H, D, batch)), "alloc");
+  return brc_warp_affine_backward_scratch(ctx, d_src, W, H, D, batch, d_params, d_grad_out, d_grad_params,
+                                          d_grad_src, ctx->partials.ptr, ctx->partials.bytes);
+}
+
+extern "C" int brc_warp_affine_backward_scratch(brc_ctx* ctx, const float* d_src, int W, int H, int D, int batch,
+                                                const float* d_params, const float* d_grad_out,
+                                                double* d_grad_params, float* d_grad_src, void* d_scratch,
+                                                size_t scratch_bytes) {
+  if (!ctx) return BRC_ERR_INVALID;
+  if (!d_src || !d_params || !d_grad_out || !d_grad_params || W <= 0 || H <= 0 || D <= 0 || batch <= 0 ||
+      batch > 65535 || !d_scratch || (reinterpret_cast<uintptr_t>(d_scratch) & 7) != 0 ||
+      scratch_bytes < brc_warp_affine_backward_scratch_bytes(W, H, D, batch))
+    return ctx->fail(BRC_ERR_INVALID, "brc_warp_affine_backward: bad argument");
+  cudaSetDevice(ctx->device);
   const long long V = (long long)W * H * D;
   const int nblk = brc::warp_affine_backward_blocks(V);
-  BRC_TRY(ctx, ctx->partials.ensure(sizeof(double) * 12 * nblk * (size_t)batch), "alloc");
   if (d_grad_src)
     BRC_TRY(ctx, cudaMemsetAsync(d_grad_src, 0, sizeof(float) * V * batch, ctx->stream()), "memset");
-  BRC_TRY(ctx, brc::warp_affine_backward(d_src, W, H, D, batch, d_params, d_grad_out, ctx->partials.as<double>(),
-                                         nblk, d_grad_params, d_grad_src, ctx->stream()),
+  BRC_TRY(ctx, brc::warp_affine_backward(d_src, W, H, D, batch, d_params, d_grad_out,
+                                         static_cast<double*>(d_scratch), nblk, d_grad_params, d_grad_src, ctx->stream()),
           "warp_affine_backward");
   ctx->launches += 2;
   return BRC_OK;

@@ -331,10 +331,20 @@ int brc_filter3d_ssd_adjoint(brc_ctx* ctx, const float* d_residual, int W, int H
  * output gradient, with the exact derivative of the clamp-to-edge
  * trilinear interpolant; d_grad_src (may be NULL) receives dL/dsrc by
  * atomic scatter (zeroed first).  Forward: InterpolateVolumeLinearLinear
- * (kernelRegistration.cpp:1066-1101). */
+ * (kernelRegistration.cpp:1066-1101).
+ *
+ * The parameter sums go through partial rows: brc_warp_affine_backward keeps
+ * them in the context's workspace (calls on one context follow one another
+ * on the GPU, and a captured call is valid until the workspace grows),
+ * brc_warp_affine_backward_scratch in d_scratch of the caller (as
+ * brc_filter3d_ssd_scratch). */
 int brc_warp_affine_backward(brc_ctx* ctx, const float* d_src, int W, int H, int D, int batch,
                              const float* d_params, const float* d_grad_out, double* d_grad_params,
                              float* d_grad_src);
+size_t brc_warp_affine_backward_scratch_bytes(int W, int H, int D, int batch);
+int brc_warp_affine_backward_scratch(brc_ctx* ctx, const float* d_src, int W, int H, int D, int batch,
+                                     const float* d_params, const float* d_grad_out, double* d_grad_params,
+                                     float* d_grad_src, void* d_scratch, size_t scratch_bytes);
 
 /* Adjoint of brc_warp_field: dL/dfield (3 volumes, may be NULL) and
  * dL/dsrc (may be NULL, zeroed then scattered).  Forward:

@@ -238,48 +238,60 @@ def _objective_inputs(shape, seed, lin_filters):
 
 def test_objective_keeps_no_sums_in_the_shared_context(lin_filters, monkeypatch):
     """One context serves every stream of a device, so the objective may hold
-    no per-call sums in it: a field objective after a filtering and a
-    smoothing of the same volume leaves the context's workspace as it was."""
+    no per-call sums in it: a field objective, and the affine gradient, after a
+    filtering and a smoothing of the same volume leave the context's workspace
+    as it was."""
     monkeypatch.setattr(AG, "_contexts", {})
     moving, q, field = _objective_inputs((9, 12, 10), 5, lin_filters)
     before = AG._ctx(moving.device).workspace_bytes
     AG.registration_objective(moving, q, lin_filters, SIGMA, field=field)
     assert AG._ctx(moving.device).workspace_bytes == before
+    p = torch.tensor(_params(), dtype=torch.float32, device="cuda", requires_grad=True)
+    AG.warp_affine(moving[None], p.reshape(1, 12)).sum().backward()
+    assert AG._ctx(moving.device).workspace_bytes == before
 
 
-def test_objectives_on_two_streams(lin_filters):
-    """Objectives queued alternately on two streams, the large and the small
-    one of each round free to run at once, give the losses of calls that run
-    alone, bit for bit (a fixed order of sums)."""
+@pytest.mark.parametrize("form", ["field", "params"])
+def test_objectives_on_two_streams(form, lin_filters):
+    """Objectives and their gradients queued alternately on two streams, the
+    large and the small one of each round free to run at once, give the results
+    of calls that run alone, bit for bit (a fixed order of sums)."""
     cases = [_objective_inputs(s, i, lin_filters) for i, s in enumerate([(40, 64, 64), (12, 20, 16)])]
+
+    def step(m, q, f):
+        x = (f if form == "field" else torch.tensor(_params(), dtype=torch.float32, device="cuda")).requires_grad_(True)
+        loss = AG.registration_objective(m, q, lin_filters, SIGMA, **{form: x})
+        return torch.cat([loss.detach().reshape(1), torch.autograd.grad(loss, x)[0].reshape(-1)])
+
     alone = []
-    for m, q, f in cases:
-        alone.append(AG.registration_objective(m, q, lin_filters, SIGMA, field=f))
+    for c in cases:
+        alone.append(step(*c))
         torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in cases]
     for s in streams:
         s.wait_stream(torch.cuda.current_stream())
-    losses = []
+    outs = []
     for _ in range(20):
         for (m, q, f), s in zip(cases, streams):
             with torch.cuda.stream(s):
-                losses.append(AG.registration_objective(m, q, lin_filters, SIGMA, field=f))
+                outs.append(step(m, q, f))
     torch.cuda.synchronize()
-    for k, loss in enumerate(losses):
-        assert torch.equal(loss, alone[k % 2])
+    for k, out in enumerate(outs):
+        assert torch.equal(out, alone[k % 2])
 
 
-def test_captured_objective_outlives_later_calls(lin_filters, monkeypatch):
-    """A field objective captured in a CUDA graph replays to the eager loss
-    and gradient after calls that make the context grow: it holds no memory
+@pytest.mark.parametrize("form", ["field", "params"])
+def test_captured_objective_outlives_later_calls(form, lin_filters, monkeypatch):
+    """An objective and its gradient captured in a CUDA graph replay to the
+    eager results after calls that make the context grow: they hold no memory
     of the context."""
     monkeypatch.setattr(AG, "_contexts", {})
     m, q, f = _objective_inputs((10, 14, 12), 3, lin_filters)
-    f.requires_grad_(True)
+    x = (f if form == "field" else torch.tensor(_params(), dtype=torch.float32, device="cuda")).requires_grad_(True)
 
     def step():
-        loss = AG.registration_objective(m, q, lin_filters, SIGMA, field=f)
-        return (loss.detach(),) + torch.autograd.grad(loss, f)
+        loss = AG.registration_objective(m, q, lin_filters, SIGMA, **{form: x})
+        return (loss.detach(),) + torch.autograd.grad(loss, x)
 
     eager = step()
     stream = torch.cuda.Stream()
@@ -293,6 +305,7 @@ def test_captured_objective_outlives_later_calls(lin_filters, monkeypatch):
     m2, q2, _ = _objective_inputs((40, 64, 64), 4, lin_filters)
     p = torch.tensor(_params(), dtype=torch.float32, device="cuda", requires_grad=True)
     AG.registration_objective(m2, q2, lin_filters, SIGMA, params=p).backward()
+    AG._ctx(m.device).register_linear(m2, m2[None].repeat(8, 1, 1, 1), lin_filters, 1)  # larger partial rows
     g.replay()
     torch.cuda.synchronize()
     for a, b in zip(captured, eager):
