@@ -13,6 +13,8 @@ forward and backward passes are the library's CUDA kernels.
 `registration_objective` composes them into the filter-response SSD of a
 moving volume, warped by 12 affine parameters or a displacement field,
 against a reference: L = sum_k sum_x |q_k(warp(S moving)) - q_k(S ref)|^2.
+Where the reference responses are constants, filtering, residual and sum of
+squares are one fused operation (FilterSsd).
 The reference responses are computed once and kept (a checkpoint per
 scale when used in a pyramid); torch only holds tensors and stitches the
 graph together.
@@ -23,6 +25,8 @@ import ctypes
 
 import numpy as np
 import torch
+from torch.autograd.forward_ad import unpack_dual
+from torch.autograd.function import once_differentiable
 
 from . import _lib as L
 from .api import Context, _check, _host_filters, _p
@@ -146,7 +150,9 @@ class Filter3d(torch.autograd.Function):
 
 class FilterSsd(torch.autograd.Function):
     """Real volumes (B,D,H,W) and reference responses (B,nfilt,D,H,W,2) ->
-    sum of squared response differences."""
+    sum of squared response differences.  First derivatives only: a second
+    backward pass raises (the residual is kept as a value, without its
+    dependence on the responses)."""
 
     @staticmethod
     def forward(fctx, vol, filters, q_ref):
@@ -168,6 +174,7 @@ class FilterSsd(torch.autograd.Function):
         return loss
 
     @staticmethod
+    @once_differentiable
     def backward(fctx, g):
         res, = fctx.saved_tensors
         c = _ctx(res.device)
@@ -215,10 +222,17 @@ def registration_objective(moving: torch.Tensor, q_ref: torch.Tensor, filters, s
         w = warp_affine(s, params.reshape(1, 12))
     else:
         w = warp_field(s[0], field)[None]
-    # one fused pass where the reference responses have the responses' own
-    # layout; anything that broadcasts or converts goes through torch
-    if (isinstance(q_ref, torch.Tensor) and q_ref.dtype == torch.float32 and q_ref.device == w.device
-            and tuple(q_ref.shape) == (w.shape[0], len(filters)) + tuple(w.shape[1:]) + (2,)):
+    if _fusable(q_ref, w, len(filters)):
         return FilterSsd.apply(w, filters, q_ref)
     q = filter3d(w, filters)
     return ((q - q_ref) ** 2).sum()
+
+
+def _fusable(q_ref, w: torch.Tensor, nfilt: int) -> bool:
+    """The objective of the warped volumes w takes the fused pass where the
+    reference responses are constants in the responses' own layout.  What
+    broadcasts, converts or is differentiated (of any order, or by forward-mode
+    tangents) goes through torch."""
+    return (isinstance(q_ref, torch.Tensor) and q_ref.dtype == torch.float32 and q_ref.device == w.device
+            and tuple(q_ref.shape) == (w.shape[0], nfilt) + tuple(w.shape[1:]) + (2,)
+            and not (q_ref.requires_grad and torch.is_grad_enabled()) and unpack_dual(q_ref).tangent is None)

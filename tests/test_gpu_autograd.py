@@ -206,9 +206,10 @@ def test_filter_adjoint_tile_edges(shape, nf, offset, bank):
 def test_objective_equals_its_torch_form(shape, offset, lin_filters):
     """The fused residual and sum of squares against the same objective from
     the filtering and torch's elementwise operations: loss, gradient of the
-    parameters and of the reference responses, with reference responses that
-    are 16-byte aligned and that are not.  Both sum FP32 squares of the same
-    residuals in another order: 1e-5 relative."""
+    parameters and of the reference responses (FilterSsd itself; the objective
+    takes the torch form for these), with reference responses that are 16-byte
+    aligned and that are not.  Both sum FP32 squares of the same residuals in
+    another order: 1e-5 relative.  A second backward pass raises."""
     gen = torch.Generator().manual_seed(sum(shape))
     moving = (torch.randn(shape, generator=gen) * 50 + 100).cuda()
     q = AG.reference_responses((torch.randn(shape, generator=gen) * 50 + 100).cuda(), lin_filters, SIGMA)
@@ -217,12 +218,18 @@ def test_objective_equals_its_torch_form(shape, offset, lin_filters):
     grads = []
     for fused in (True, False):
         p = torch.tensor(_params(), dtype=torch.float32, device="cuda", requires_grad=True)
-        q_ref = buf[offset:].reshape(q.shape).detach().requires_grad_(True)
+        q_ref = buf[offset:].reshape(q.shape).detach()
         if fused:
-            loss = AG.registration_objective(moving, q_ref, lin_filters, SIGMA, params=p)
-        else:
-            w = AG.warp_affine(AG.smooth3d(moving[None], SIGMA), p.reshape(1, 12))
-            loss = ((AG.filter3d(w, lin_filters) - q_ref) ** 2).sum()
+            objective = AG.registration_objective(moving, q_ref, lin_filters, SIGMA, params=p).detach()
+        q_ref.requires_grad_(True)
+        w = AG.warp_affine(AG.smooth3d(moving[None], SIGMA), p.reshape(1, 12))
+        loss = AG.FilterSsd.apply(w, lin_filters, q_ref) if fused else ((AG.filter3d(w, lin_filters) - q_ref) ** 2).sum()
+        if fused:
+            assert torch.equal(loss.detach(), objective)
+            g, = torch.autograd.grad(torch.sqrt(loss), q_ref, create_graph=True)
+            with pytest.raises(RuntimeError, match="once_differentiable"):
+                g.sum().backward()
+            loss = AG.FilterSsd.apply(w, lin_filters, q_ref)
         grads.append((loss.detach(),) + torch.autograd.grad(3.0 * loss, (p, q_ref)))
     for a, b in zip(*grads):
         assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max())
