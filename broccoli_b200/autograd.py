@@ -29,7 +29,7 @@ from torch.autograd.forward_ad import unpack_dual
 from torch.autograd.function import once_differentiable
 
 from . import _lib as L
-from .api import Context, _check, _host_filters, _p
+from .api import Context, _check, _host_filters, _p, _vol_batch
 
 # One context per device, shared by all its streams: an operation that needs
 # memory during its call takes torch's, on its own stream.
@@ -156,10 +156,14 @@ class FilterSsd(torch.autograd.Function):
 
     @staticmethod
     def forward(fctx, vol, filters, q_ref):
-        c = _ctx(vol.device)
+        v = _vol_batch(vol)
         f = _host_filters(filters)
-        v = vol.contiguous()
         B, D, H, W = v.shape
+        if not isinstance(q_ref, torch.Tensor) or q_ref.dtype != torch.float32 or q_ref.device != v.device:
+            raise TypeError("reference responses must be float32 tensors on the volumes' device")
+        if tuple(q_ref.shape) != (B, f.shape[0], D, H, W, 2):
+            raise ValueError("reference responses must have shape (B, nfilt, D, H, W, 2)")
+        c = _ctx(v.device)
         r = q_ref.detach().contiguous()
         res = torch.empty_like(r)
         loss = torch.empty((), dtype=torch.float32, device=v.device)
@@ -170,6 +174,7 @@ class FilterSsd(torch.autograd.Function):
         _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), f.shape[0], _p(r), _p(res),
                      _p(loss), _p(sums), size))
         fctx.filters = f
+        fctx.vol_shape = vol.shape
         fctx.save_for_backward(res)
         return loss
 
@@ -183,7 +188,7 @@ class FilterSsd(torch.autograd.Function):
         gl = g.contiguous().to(torch.float32)
         gv = None
         if fctx.needs_input_grad[0]:
-            gv = torch.empty((B, D, H, W), dtype=torch.float32, device=res.device)
+            gv = torch.empty(fctx.vol_shape, dtype=torch.float32, device=res.device)
             fn = _sig("brc_filter3d_ssd_adjoint", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P])
             _check(c, fn(c.handle, _p(res), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), nf, _p(gl), _p(gv)))
         return gv, None, (-2.0 * gl) * res if fctx.needs_input_grad[2] else None

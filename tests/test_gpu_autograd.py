@@ -317,3 +317,18 @@ def test_captured_objective_outlives_later_calls(form, lin_filters, monkeypatch)
     torch.cuda.synchronize()
     for a, b in zip(captured, eager):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("vol, ref, error", [
+    (torch.float64, torch.float32, TypeError), (torch.float16, torch.float32, TypeError),
+    (torch.float32, torch.float64, TypeError), (torch.float32, torch.float16, TypeError),
+    (torch.float32, "cpu", TypeError), (torch.float32, "short", ValueError)])
+def test_fused_objective_refuses_what_the_kernels_cannot_read(vol, ref, error, lin_filters):
+    """Types, devices and shapes of the fused operation's inputs, refused
+    before their pointers are used."""
+    shape = (5, 6, 8)
+    v = torch.zeros((1,) + shape, device="cuda", dtype=vol)
+    q = torch.zeros((1, 3) + shape + (2,), device="cpu" if ref == "cpu" else "cuda")
+    q = q[:, :2] if ref == "short" else q.to(ref) if isinstance(ref, torch.dtype) else q
+    with pytest.raises(error):
+        AG.FilterSsd.apply(v, lin_filters, q)

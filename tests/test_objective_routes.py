@@ -1,6 +1,7 @@
 """The route of the differentiable objective on the CPU: smoothing, warp and
 filtering replaced by torch expressions, so that only the choice between the
 fused pass and the torch form of the sum of squares is the package's."""
+import numpy as np
 import pytest
 import torch
 from torch.autograd import forward_ad
@@ -70,3 +71,13 @@ def test_forward_mode_tangents_of_the_reference_responses(stages):
         q = forward_ad.make_dual(q_ref, t)
         got, want = (forward_ad.unpack_dual(o(moving, q)).tangent for o in (_objective, _plain))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.float16])
+def test_fused_objective_refuses_host_tensors(dtype):
+    """The fused operation hands raw pointers to the library: tensors that are
+    not float32 on CUDA are refused before that, whatever the device."""
+    bank = np.zeros((3, 2, 7, 7, 7), np.float32)
+    vol = torch.zeros((1,) + SHAPE, dtype=dtype)
+    with pytest.raises(TypeError):
+        AG.FilterSsd.apply(vol, bank, torch.zeros((1, 3) + SHAPE + (2,), dtype=dtype))
