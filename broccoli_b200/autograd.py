@@ -181,7 +181,11 @@ class FilterSsd(torch.autograd.Function):
     @staticmethod
     @once_differentiable
     def backward(fctx, g):
+        # saved-tensor hooks may give the residual back in another layout or type
         res, = fctx.saved_tensors
+        if res.device != g.device:
+            raise TypeError("the saved residual must be on the gradient's device")
+        res = res.to(torch.float32).contiguous()
         c = _ctx(res.device)
         f = fctx.filters
         B, nf, D, H, W, _ = res.shape

@@ -332,3 +332,19 @@ def test_fused_objective_refuses_what_the_kernels_cannot_read(vol, ref, error, l
     q = q[:, :2] if ref == "short" else q.to(ref) if isinstance(ref, torch.dtype) else q
     with pytest.raises(error):
         AG.FilterSsd.apply(v, lin_filters, q)
+
+
+@pytest.mark.parametrize("unpack", [lambda t: t.movedim(1, -1).contiguous().movedim(-1, 1), lambda t: t.double()])
+def test_fused_objective_under_saved_tensor_hooks(unpack, lin_filters):
+    """A saved-tensor hook that gives the residual back with other strides, or
+    in float64, changes neither gradient of the fused operation."""
+    m, q, _ = _objective_inputs((5, 6, 8), 6, lin_filters)
+    grads = []
+    for hook in (lambda t: t, unpack):
+        v = m[None].clone().requires_grad_(True)
+        r = q.clone().requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.clone(), hook):
+            loss = AG.FilterSsd.apply(v, lin_filters, r)
+        grads.append(torch.autograd.grad(loss, (v, r)))
+    for a, b in zip(*grads):
+        assert torch.equal(a, b)
