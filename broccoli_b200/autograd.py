@@ -240,8 +240,10 @@ def registration_objective(moving: torch.Tensor, q_ref: torch.Tensor, filters, s
 def _fusable(q_ref, w: torch.Tensor, nfilt: int) -> bool:
     """The objective of the warped volumes w takes the fused pass where the
     reference responses are constants in the responses' own layout.  What
-    broadcasts, converts or is differentiated (of any order, or by forward-mode
-    tangents) goes through torch."""
-    return (isinstance(q_ref, torch.Tensor) and q_ref.dtype == torch.float32 and q_ref.device == w.device
+    broadcasts, converts, has operations of its own (subclasses, sparse
+    layouts) or is differentiated (of any order, or by forward-mode tangents)
+    goes through torch."""
+    return (type(q_ref) in (torch.Tensor, torch.nn.Parameter) and q_ref.layout == torch.strided
+            and q_ref.dtype == torch.float32 and q_ref.device == w.device
             and tuple(q_ref.shape) == (w.shape[0], nfilt) + tuple(w.shape[1:]) + (2,)
             and not (q_ref.requires_grad and torch.is_grad_enabled()) and unpack_dual(q_ref).tangent is None)

@@ -81,3 +81,23 @@ def test_fused_objective_refuses_host_tensors(dtype):
     vol = torch.zeros((1,) + SHAPE, dtype=dtype)
     with pytest.raises(TypeError):
         AG.FilterSsd.apply(vol, bank, torch.zeros((1, 3) + SHAPE + (2,), dtype=dtype))
+
+
+class Halved(torch.Tensor):
+    """Responses stored at twice their value: subtraction reads the half."""
+
+    @classmethod
+    def __torch_function__(cls, func, types, args=(), kwargs=None):
+        plain = [a.as_subclass(torch.Tensor) if isinstance(a, Halved) else a for a in args]
+        if func in (torch.Tensor.sub, torch.Tensor.__sub__, torch.sub):
+            plain[1] = 0.5 * plain[1]
+        return func(*plain, **(kwargs or {}))
+
+
+def test_reference_responses_with_operations_of_their_own(stages):
+    """Tensor subclasses and sparse tensors take the torch form, which calls
+    their operations."""
+    moving, q_ref = _inputs()
+    want = _plain(moving, q_ref)
+    assert torch.equal(_objective(moving, (2.0 * q_ref).as_subclass(Halved)), want)
+    assert torch.equal(_objective(moving, q_ref.to_sparse()), want)
