@@ -108,6 +108,17 @@ class Context:
         _check(self, L.lib().brc_selftest_phase_atan2(self.handle, _p(y), _p(x), _p(out), y.numel()))
         return out
 
+    def selftest_filter_shape(self, shape, batch: int, filters, precision: int = L.PREC_FP32, set: int = 0) -> int:
+        """The launch shape that an FP32 filtering of `batch` volumes of
+        `shape` (D, H, W) takes; set > 0 fixes it first."""
+        f = _host_filters(filters)
+        D, H, W = shape
+        used = ctypes.c_int()
+        self._bind_stream()
+        _check(self, L.lib().brc_selftest_filter_shape(self.handle, W, H, D, batch, f.ctypes.data_as(ctypes.c_void_p),
+                                                       f.shape[0], precision, set, ctypes.byref(used)))
+        return used.value
+
     # ---- kernels ---------------------------------------------------------
 
     def filter3d(self, vol: torch.Tensor, filters, precision: int = L.PREC_FP32) -> torch.Tensor:

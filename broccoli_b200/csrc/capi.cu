@@ -52,6 +52,12 @@ static int timed_volumes(long long V, int batch) {
   return nb;
 }
 
+// The tuner's key of the FP32 filtering.
+static std::tuple<int, int, int, int, int> fp32_key(brc::FilterKind kind, int nfilt, int W, int H, int D,
+                                                    int batch) {
+  return {nfilt + (kind == brc::kFilterSym ? 100 : 0), W, H, D, timed_volumes((long long)W * H * D, batch)};
+}
+
 static bool bad_dims(int W, int H, int D) {
   return W <= 0 || H <= 0 || D <= 0 || (long long)W * H * D > (1ll << 31);
 }
@@ -214,8 +220,8 @@ int brc_ctx::smooth(const float* vol, int W, int H, int D, int batch, const floa
 
 int brc_ctx::tune_fp32(const float* bank, brc::FilterKind kind, int nfilt, int W, int H, int D, int batch, int* tz) {
   const long long V = (long long)W * H * D;
-  const int nb = timed_volumes(V, batch);
-  const auto key = std::make_tuple(nfilt + (kind == brc::kFilterSym ? 100 : 0), W, H, D, nb);
+  const auto key = fp32_key(kind, nfilt, W, H, D, batch);
+  const int nb = std::get<4>(key);
   auto it = fp32_tuned.find(key);
   if (it != fp32_tuned.end()) {
     *tz = it->second;
@@ -224,7 +230,23 @@ int brc_ctx::tune_fp32(const float* bank, brc::FilterKind kind, int nfilt, int W
   *tz = brc::filter3d_default_tz(D);
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   BRC_TRY(this, cudaStreamIsCapturing(stream(), &cap), "capture status");
-  if (cap != cudaStreamCaptureStatusNone) return BRC_OK;  // no timing inside a capture
+  if (cap != cudaStreamCaptureStatusNone) {
+    // no timing inside a capture: the choice timed for the nearest launch size
+    // of this shape, so that one call outside captures serves them all
+    // (the larger of two equally near; none timed: the untimed choice)
+    double best = -1.0;
+    for (auto& t : fp32_tuned) {
+      if (std::tie(std::get<0>(t.first), std::get<1>(t.first), std::get<2>(t.first), std::get<3>(t.first)) !=
+          std::tie(std::get<0>(key), std::get<1>(key), std::get<2>(key), std::get<3>(key)))
+        continue;
+      const double ratio = (double)std::get<4>(t.first) / nb, far = ratio < 1.0 ? 1.0 / ratio : ratio;
+      if (best < 0.0 || far <= best) {
+        best = far;
+        *tz = t.second;
+      }
+    }
+    return BRC_OK;
+  }
   int cand[8];
   const int n = brc::filter3d_tz_candidates(nfilt, cand, 8);
   // time each z depth on zero-filled scratch volumes (the kernels' work does
@@ -410,6 +432,27 @@ int brc_selftest_phase_atan2(brc_ctx* ctx, const float* d_y, const float* d_x, f
   BRC_TRY(ctx, brc::phase_atan2_eval(d_y, d_x, d_out, n, ctx->stream()), "phase_atan2");
   ctx->launches += n > 0 ? 1 : 0;
   return BRC_OK;
+}
+
+int brc_selftest_filter_shape(brc_ctx* ctx, int W, int H, int D, int batch, const float* h_filters, int nfilt,
+                              int precision, int set, int* used) {
+  BRC_CHECK_CTX(ctx);
+  if (!used || !h_filters || bad_dims(W, H, D) || batch <= 0 || (nfilt != 3 && nfilt != 6) || set < 0 ||
+      (precision != BRC_PREC_FP32 && precision != BRC_PREC_FP32_GENERAL))
+    return ctx->fail(BRC_ERR_INVALID, "brc_selftest_filter_shape: bad argument");
+  cudaSetDevice(ctx->device);
+  FilterPath fp;
+  if (set > 0) {
+    int cand[8];
+    const int n = brc::filter3d_tz_candidates(nfilt, cand, 8);
+    if (std::find(cand, cand + n, set) == cand + n)
+      return ctx->fail(BRC_ERR_INVALID, "brc_selftest_filter_shape: no such shape");
+    const auto kind = brc::filter3d_pack(h_filters, nfilt, precision == BRC_PREC_FP32, fp.bank);
+    ctx->fp32_tuned[fp32_key(kind, nfilt, W, H, D, batch)] = set;
+  }
+  const int s = make_filter_path(ctx, h_filters, nfilt, precision, W, H, D, batch, &fp);
+  if (s == BRC_OK) *used = fp.tz;
+  return s;
 }
 
 size_t brc_ctx_workspace_bytes(const brc_ctx* ctx) { return ctx ? ctx->workspace() : 0; }

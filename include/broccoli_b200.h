@@ -369,6 +369,17 @@ int brc_selftest_bounded_wait(brc_ctx* ctx, int wait_ms);
  * (kernelRegistration.cpp:173-382). */
 int brc_selftest_phase_atan2(brc_ctx* ctx, const float* d_y, const float* d_x, float* d_out, long long n);
 
+/* The launch shape of the FP32 filtering, which the context picks by timing
+ * (every shape gives the same responses bit for bit), so that each can be
+ * tested.  set > 0 fixes the shape of brc_filter3d for this bank kind, volume
+ * and batch (sizes count by powers of two) as the timing would have
+ * (BRC_ERR_INVALID if it is none of the kernels' shapes); *used receives the
+ * shape such a call takes now (timed first where none is known and the
+ * stream is not being captured).  precision: BRC_PREC_FP32 or
+ * BRC_PREC_FP32_GENERAL.  No counterpart in the reference. */
+int brc_selftest_filter_shape(brc_ctx* ctx, int W, int H, int D, int batch, const float* h_filters, int nfilt,
+                              int precision, int set, int* used);
+
 /* ---- device memory and host copies (for hosts without a CUDA runtime) --- */
 
 /* cudaMalloc / cudaFree on the context's device.  Replaces the clCreateBuffer

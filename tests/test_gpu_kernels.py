@@ -10,6 +10,7 @@ import torch
 from conftest import rel_err
 from broccoli_b200 import _lib as L
 from broccoli_b200 import filters as F
+from broccoli_b200.api import Context
 
 pytestmark = pytest.mark.gpu
 TOL = 1e-4
@@ -225,3 +226,27 @@ def test_smoothing_tile_edges_vs_oracle(ctx, orc, shape, weighted):
         ref = [orc.smooth3d(v, *taps) for v in vols]
     for b in range(2):
         assert rel_err(got[b], ref[b]) < TOL
+
+
+def test_filter_shape_inside_a_capture(lin_filters):
+    """A capture cannot time: it takes the launch shape known for the nearest
+    launch size of the volume shape (powers of two, the larger of two equally
+    near), and the untimed one where none is known.  One warm call outside thus
+    serves captures of every batch."""
+    c = Context(0)
+    shape = (9, 11, 13)
+    vols = torch.rand((4,) + shape, device="cuda")
+    c.filter3d(vols, lin_filters)  # loads the kernels; times launches of 4
+    with torch.cuda.graph(torch.cuda.CUDAGraph()):
+        c.filter3d(vols, lin_filters)
+        other = c.selftest_filter_shape((9, 11, 14), 4, lin_filters)
+    assert other == 3  # the depth that divides 9 planes
+    for known, queries in [({4: 8}, {1: 8, 3: 8, 7: 8, 200: 8}), ({1: 6}, {1: 6, 2: 8, 4: 8}),
+                           ({16: 2}, {2: 8, 7: 8, 8: 2, 40: 2})]:
+        for batch, shape_code in known.items():
+            assert c.selftest_filter_shape(shape, batch, lin_filters, set=shape_code) == shape_code
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            c.filter3d(vols, lin_filters)
+            got = {batch: c.selftest_filter_shape(shape, batch, lin_filters) for batch in queries}
+        assert got == queries
+    c.close()
