@@ -163,12 +163,14 @@ __device__ __forceinline__ void floor_small(float v, float& f, int& i) {
 // clamp-to-edge addressing, exact float weights (the sampler of
 // kernelRegistration.cpp:1064).  u, v, w include the +0.5 texel offset.
 //
-// A warp whose eight neighbours are all inside the volume takes one base
-// address and constant offsets; any other warp clamps every index, without a
-// branch per lane (at W = 64 every warp of a moved volume holds an edge, and
-// lanes that took two paths one after the other doubled its instructions).
+// The lanes of `mask` (those of the warp that sample at all, the same value on
+// each of them) choose together: where the eight neighbours of every one are
+// inside the volume they take one base address and constant offsets, else
+// they all clamp every index (at W = 64 every warp of a moved volume holds an
+// edge, and lanes that took two paths one after the other doubled its
+// instructions).  Every lane of the mask comes to the vote once per call.
 __device__ __forceinline__ float sample_linear(const float* __restrict__ T, int W, int H, int D,
-                                              float u, float v, float w) {
+                                              float u, float v, float w, unsigned mask) {
   // volumes hold fewer than 2^31 voxels (checked by the launchers)
   const float uu = u - 0.5f, vv = v - 0.5f, ww = w - 0.5f;
   float fu, fv, fw;
@@ -189,8 +191,8 @@ __device__ __forceinline__ float sample_linear(const float* __restrict__ T, int 
   const int WH = W * H;
   float t000, t100, t010, t110, t001, t101, t011, t111;
   const bool inside =
-      (unsigned)i0 < (unsigned)(W - 1) && (unsigned)j0 < (unsigned)(H - 1) && (unsigned)k0 < (unsigned)(D - 1);
-  if (__all_sync(__activemask(), inside)) {
+      ((unsigned)i0 < (unsigned)(W - 1)) & ((unsigned)j0 < (unsigned)(H - 1)) & ((unsigned)k0 < (unsigned)(D - 1));
+  if (__all_sync(mask, inside)) {
     const float* p0 = T + (i0 + j0 * W + k0 * WH);
     const float* p1 = p0 + WH;
     t000 = __ldg(p0);
@@ -246,19 +248,33 @@ __device__ __forceinline__ void load_clamped(const float* __restrict__ T, int W,
   t[7] = __ldg(T + (x1 + r11));
 }
 
+// sample_linear of one lane, for positions of any size.
+__device__ __forceinline__ float sample_clamped(const float* __restrict__ T, int W, int H, int D, float u, float v,
+                                                float w) {
+  const float uu = u - 0.5f, vv = v - 0.5f, ww = w - 0.5f;
+  const float fu = floorf(uu), fv = floorf(vv), fw = floorf(ww);
+  const float a = uu - fu, b = vv - fv, c = ww - fw;
+  float t[8];
+  load_clamped(T, W, H, D, (int)fu, (int)fv, (int)fw, t);
+#pragma unroll
+  for (int q = 0; q < 8; q += 2) t[q] = fmaf(a, t[q + 1] - t[q], t[q]);
+  t[0] = fmaf(b, t[2] - t[0], t[0]);
+  t[4] = fmaf(b, t[6] - t[4], t[4]);
+  return fmaf(c, t[4] - t[0], t[0]);
+}
+
 // sample_linear at two positions at once (the halves of u, v, w), the
 // arithmetic as packed pairs: the same operations in the same order per half.
+// One vote, as there; a lane with a position that floor_small does not take
+// votes against the unclamped loads.
 __device__ __forceinline__ float2 sample_linear_pair(const float* __restrict__ T, int W, int H, int D, F2 u, F2 v,
-                                                     F2 w) {
+                                                     F2 w, unsigned mask) {
   const F2 half = f2_twice(0.5f), magic = f2_twice(12582912.0f);
   const F2 uu = f2_sub(u, half), vv = f2_sub(v, half), ww = f2_sub(w, half);
   const float2 us = f2_unpack(uu), vs = f2_unpack(vv), ws = f2_unpack(ww);
   const float far = fmaxf(fmaxf(fmaxf(fabsf(us.x), fabsf(us.y)), fmaxf(fabsf(vs.x), fabsf(vs.y))),
                           fmaxf(fabsf(ws.x), fabsf(ws.y)));
-  if (!(far < 4194304.0f)) {
-    const float2 u2 = f2_unpack(u), v2 = f2_unpack(v), w2 = f2_unpack(w);
-    return make_float2(sample_linear(T, W, H, D, u2.x, v2.x, w2.x), sample_linear(T, W, H, D, u2.y, v2.y, w2.y));
-  }
+  const bool near = far < 4194304.0f;
   // floor_small of the six coordinates
   const F2 tu = f2_add_rm(uu, magic), tv = f2_add_rm(vv, magic), tw = f2_add_rm(ww, magic);
   const F2 a = f2_sub(uu, f2_sub(tu, magic)), b = f2_sub(vv, f2_sub(tv, magic)), c = f2_sub(ww, f2_sub(tw, magic));
@@ -267,10 +283,10 @@ __device__ __forceinline__ float2 sample_linear_pair(const float* __restrict__ T
   const int ja = __float_as_int(iv.x) - 0x4B400000, jb = __float_as_int(iv.y) - 0x4B400000;
   const int ka = __float_as_int(iw.x) - 0x4B400000, kb = __float_as_int(iw.y) - 0x4B400000;
   float ta[8], tb[8];
-  const bool inside = (unsigned)ia < (unsigned)(W - 1) && (unsigned)ja < (unsigned)(H - 1) &&
-                      (unsigned)ka < (unsigned)(D - 1) && (unsigned)ib < (unsigned)(W - 1) &&
-                      (unsigned)jb < (unsigned)(H - 1) && (unsigned)kb < (unsigned)(D - 1);
-  if (__all_sync(__activemask(), inside)) {
+  const bool inside = near & ((unsigned)ia < (unsigned)(W - 1)) & ((unsigned)ja < (unsigned)(H - 1)) &
+                      ((unsigned)ka < (unsigned)(D - 1)) & ((unsigned)ib < (unsigned)(W - 1)) &
+                      ((unsigned)jb < (unsigned)(H - 1)) & ((unsigned)kb < (unsigned)(D - 1));
+  if (__all_sync(mask, inside)) {
     const long long WH = (long long)W * H;
     const float* pa = T + (ia + (ja + ka * H) * W);
     const float* pb = T + (ib + (jb + kb * H) * W);
@@ -280,9 +296,12 @@ __device__ __forceinline__ float2 sample_linear_pair(const float* __restrict__ T
       ta[q] = __ldg(pa + o + (q & 1));
       tb[q] = __ldg(pb + o + (q & 1));
     }
-  } else {
+  } else if (near) {
     load_clamped(T, W, H, D, ia, ja, ka, ta);
     load_clamped(T, W, H, D, ib, jb, kb, tb);
+  } else {
+    const float2 u2 = f2_unpack(u), v2 = f2_unpack(v), w2 = f2_unpack(w);
+    return make_float2(sample_clamped(T, W, H, D, u2.x, v2.x, w2.x), sample_clamped(T, W, H, D, u2.y, v2.y, w2.y));
   }
   F2 t[8];
 #pragma unroll
@@ -298,19 +317,21 @@ __device__ __forceinline__ float2 sample_linear_pair(const float* __restrict__ T
 // centre) with p = {t, A - I} (InterpolateVolumeLinearLinear,
 // kernelRegistration.cpp:1066-1101).
 __device__ __forceinline__ float affine_sample(const float* __restrict__ src, int W, int H, int D,
-                                               const float* __restrict__ p, int x, int y, int z) {
+                                               const float* __restrict__ p, int x, int y, int z,
+                                               unsigned mask) {
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
   const float zf = (float)z - ((float)D - 1.0f) * 0.5f;
   const float u = (float)x + p[0] + p[3] * xf + p[4] * yf + p[5] * zf + 0.5f;
   const float v = (float)y + p[1] + p[6] * xf + p[7] * yf + p[8] * zf + 0.5f;
   const float w = (float)z + p[2] + p[9] * xf + p[10] * yf + p[11] * zf + 0.5f;
-  return sample_linear(src, W, H, D, u, v, w);
+  return sample_linear(src, W, H, D, u, v, w, mask);
 }
 
 // affine_sample of voxels (x, y, z) and (x, y, z2), the same bits.
 __device__ __forceinline__ float2 affine_sample_pair(const float* __restrict__ src, int W, int H, int D,
-                                                     const float* __restrict__ p, int x, int y, int z, int z2) {
+                                                     const float* __restrict__ p, int x, int y, int z, int z2,
+                                                     unsigned mask) {
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
   const F2 zz = f2_pack((float)z, (float)z2);
@@ -323,7 +344,7 @@ __device__ __forceinline__ float2 affine_sample_pair(const float* __restrict__ s
   const F2 u = f2_add(f2_fma(f2_pack(p[5], p[5]), zf, f2_pack(pu, pu)), half);
   const F2 v = f2_add(f2_fma(f2_pack(p[8], p[8]), zf, f2_pack(pv, pv)), half);
   const F2 w = f2_add(f2_fma(f2_pack(p[11], p[11]), zf, pw), half);
-  return sample_linear_pair(src, W, H, D, u, v, w);
+  return sample_linear_pair(src, W, H, D, u, v, w, mask);
 }
 
 }  // namespace brc

@@ -949,7 +949,9 @@ warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, i
   // tiles, groups of planes, a share of the instances: blockIdx.z, + gridDim.z, ...)
   const int ty = blockIdx.x / ntx, tx = blockIdx.x - ty * ntx;
   const int x = tx * 32 + threadIdx.x, y = ty * 8 + threadIdx.y, z = NZ * blockIdx.y;
-  if (x >= W || y >= H) return;
+  const bool on = (x < W) & (y < H);
+  const unsigned mask = __ballot_sync(0xffffffffu, on);  // the sampler's lanes
+  if (!on) return;
   const int z2 = min(z + 1, D - 1);
   const long long WH = (long long)W * H;
   const int n = active_count(act, batch);
@@ -975,11 +977,11 @@ warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, i
     const float* s = src + (long long)b * src_stride;
     float* ob = o + (long long)b * out_stride;
     if constexpr (NZ == 2) {
-      const float2 r = affine_sample_pair(s, W, H, D, p, x, y, z, z2);
+      const float2 r = affine_sample_pair(s, W, H, D, p, x, y, z, z2, mask);
       ob[0] = r.x;
       if (z + 1 < D) ob[WH] = r.y;
     } else {
-      ob[0] = affine_sample(s, W, H, D, p, x, y, z);
+      ob[0] = affine_sample(s, W, H, D, p, x, y, z, mask);
     }
   }
 }
@@ -992,6 +994,7 @@ warp_field_kernel(const float* __restrict__ src, int W, int H, int D, const floa
                   long long src_stride, long long field_stride, long long out_stride) {
   const int V = W * H * D;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned mask = __ballot_sync(0xffffffffu, i < V);  // the sampler's lanes
   if (i >= V) return;
   // instance blockIdx.y
   const long long b = blockIdx.y;
@@ -1003,7 +1006,7 @@ warp_field_kernel(const float* __restrict__ src, int W, int H, int D, const floa
   int x, y, z;
   voxel_of(i, W, H, x, y, z);
   out[i] = sample_linear(src, W, H, D, (float)x + dx[i] + 0.5f, (float)y + dy[i] + 0.5f,
-                         (float)z + dz[i] + 0.5f);
+                         (float)z + dz[i] + 0.5f, mask);
 }
 
 // Linear resample with spacing (N-1)/(N'-1) (RescaleVolumeLinear,
@@ -1013,10 +1016,11 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
                       int W2, int H2, int D2, float vx, float vy, float vz) {
   const int V2 = W2 * H2 * D2;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned mask = __ballot_sync(0xffffffffu, i < V2);  // the sampler's lanes
   if (i >= V2) return;
   int x, y, z;
   voxel_of(i, W2, H2, x, y, z);
-  out[i] = sample_linear(src, W, H, D, x * vx + 0.5f, y * vy + 0.5f, z * vz + 0.5f);
+  out[i] = sample_linear(src, W, H, D, x * vx + 0.5f, y * vy + 0.5f, z * vz + 0.5f, mask);
 }
 
 // ---------------------------------------------------------------------------

@@ -143,6 +143,40 @@ def test_warp_affine_pairs_of_planes(ctx, shape):
         assert (out[b] - ref).abs().max() <= tol
 
 
+@pytest.mark.parametrize("shape", [(3, 5, 7), (4, 9, 33), (2, 8, 65), (5, 64, 64)])
+@pytest.mark.parametrize("far", [0.4, 5e6, -3e9, float("inf"), float("nan")])
+def test_warp_field_lanes_of_a_warp_mixed(ctx, shape, far):
+    """Lanes of one warp whose positions are inside, outside, beyond the small
+    floor, infinite or NaN, in a random mixture (and warps with lanes past the
+    volume's end), give what a field of one kind alone gives at each voxel."""
+    g = torch.Generator().manual_seed(sum(shape))
+    vol = torch.randn(shape, generator=g).cuda()
+    near = (torch.rand((3,) + shape, generator=g) - 0.5).cuda()
+    out = torch.full((3,) + shape, far, device="cuda")
+    pick = (torch.rand(shape, generator=g) < 0.5).cuda()
+    mixed = torch.where(pick, near, out)
+    a, b, m = (ctx.warp_field(vol, *f) for f in (near, out, mixed))
+    want = torch.where(pick, a, b)
+    assert torch.equal(m.isnan(), want.isnan())
+    assert torch.equal(m.nan_to_num(), want.nan_to_num())
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_warp_affine_lanes_of_a_warp_mixed(ctx, batch):
+    """A stretch of 2^23 along x about a central voxel: in every warp the lane
+    at the centre samples it, the others lie beyond the small floor on both
+    sides and take the edges.  One volume takes one plane per thread, three
+    take two."""
+    D, H, W = 40, 64, 65
+    g = torch.Generator().manual_seed(batch)
+    vol = torch.randn((batch, D, H, W), generator=g).cuda()
+    p = torch.zeros((batch, 12), device="cuda")
+    p[:, 3] = 2.0 ** 23
+    out = ctx.warp_affine(vol, p)
+    want = torch.cat([vol[..., :1].expand(-1, -1, -1, 32), vol[..., 32:33], vol[..., -1:].expand(-1, -1, -1, 32)], -1)
+    assert torch.equal(out, want)
+
+
 def test_warp_field_matches_golden(ctx, golden):
     out = ctx.warp_field(cuda(golden["moved"]), cuda(golden["field_x"]), cuda(golden["field_y"]),
                          cuda(golden["field_z"]))
