@@ -71,9 +71,9 @@ __device__ __forceinline__ float phase_atan2(float y, float x) {
   p = fmaf(p, s, 1.999261975e-01f);
   p = fmaf(p, s, -3.333307207e-01f);
   p = fmaf(p, s, 1.0f);
-  float r = p * t;
-  r = ay > ax ? 1.57079632679489662f - r : r;
-  r = x < 0.f ? 3.14159265358979324f - r : r;
+  float r = __fmul_rn(p, t);
+  r = ay > ax ? __fsub_rn(1.57079632679489662f, r) : r;
+  r = x < 0.f ? __fsub_rn(3.14159265358979324f, r) : r;
   return copysignf(r, y);
 }
 
@@ -322,13 +322,15 @@ __device__ __forceinline__ float affine_sample(const float* __restrict__ src, in
   const float xf = (float)x - ((float)W - 1.0f) * 0.5f;
   const float yf = (float)y - ((float)H - 1.0f) * 0.5f;
   const float zf = (float)z - ((float)D - 1.0f) * 0.5f;
-  const float u = (float)x + p[0] + p[3] * xf + p[4] * yf + p[5] * zf + 0.5f;
-  const float v = (float)y + p[1] + p[6] * xf + p[7] * yf + p[8] * zf + 0.5f;
-  const float w = (float)z + p[2] + p[9] * xf + p[10] * yf + p[11] * zf + 0.5f;
+  const float u = fmaf(p[5], zf, fmaf(p[4], yf, fmaf(p[3], xf, (float)x + p[0]))) + 0.5f;
+  const float v = fmaf(p[8], zf, fmaf(p[7], yf, fmaf(p[6], xf, (float)y + p[1]))) + 0.5f;
+  const float w = fmaf(p[11], zf, fmaf(p[10], yf, fmaf(p[9], xf, (float)z + p[2]))) + 0.5f;
   return sample_linear(src, W, H, D, u, v, w, mask);
 }
 
-// affine_sample of voxels (x, y, z) and (x, y, z2), the same bits.
+// affine_sample of voxels (x, y, z) and (x, y, z2): the same operations, each
+// rounded alike, so that a volume's result does not depend on which of the two
+// a launch takes.
 __device__ __forceinline__ float2 affine_sample_pair(const float* __restrict__ src, int W, int H, int D,
                                                      const float* __restrict__ p, int x, int y, int z, int z2,
                                                      unsigned mask) {

@@ -39,7 +39,7 @@ __device__ __forceinline__ void phase_diff_cert(float2 a, float2 c, float& pd, f
   const float re = __fadd_rn(__fmul_rn(a.x, c.x), __fmul_rn(a.y, c.y));
   const float im = __fsub_rn(__fmul_rn(a.y, c.x), __fmul_rn(a.x, c.y));
   pd = phase_atan2(im, re);
-  cert = 0.5f * (sqrt_approx(re * re + im * im) + re);
+  cert = 0.5f * __fadd_rn(sqrt_approx(fmaf(re, re, __fmul_rn(im, im))), re);
 }
 
 // Phase gradient from the neighbours along one axis
@@ -55,6 +55,19 @@ __device__ __forceinline__ float phase_grad(float2 a_p, float2 a_c, float2 a_m, 
   ti += c_p.y * c_c.x - c_p.x * c_c.y;
   tr += c_c.x * c_m.x + c_c.y * c_m.y;
   ti += c_c.y * c_m.x - c_c.x * c_m.y;
+  return phase_atan2(ti, tr);
+}
+
+// phase_grad with every rounding written out, for the kernel whose forms have
+// to agree bit for bit (left to the compiler, the products that fuse with an
+// addition differ from kernel to kernel).
+__device__ __forceinline__ float phase_grad_rn(float2 a_p, float2 a_c, float2 a_m, float2 c_p,
+                                               float2 c_c, float2 c_m) {
+  // p conj(o) of each pair of neighbours, summed in order
+  const auto re = [](float2 p, float2 o) { return fmaf(p.x, o.x, __fmul_rn(p.y, o.y)); };
+  const auto im = [](float2 p, float2 o) { return fmaf(p.y, o.x, -__fmul_rn(p.x, o.y)); };
+  const float tr = __fadd_rn(__fadd_rn(__fadd_rn(re(a_p, a_c), re(a_c, a_m)), re(c_p, c_c)), re(c_c, c_m));
+  const float ti = __fadd_rn(__fadd_rn(__fadd_rn(im(a_p, a_c), im(a_c, a_m)), im(c_p, c_c)), im(c_c, c_m));
   return phase_atan2(ti, tr);
 }
 
@@ -264,20 +277,28 @@ __device__ __forceinline__ float cluster_load(const float* p, int rank) {
   return v;
 }
 
+// Three-tap sum with the weights w1, w0, w1.
+__device__ __forceinline__ float smooth3(float w0, float w1, float a, float b, float c) {
+  return fmaf(w1, c, fmaf(w1, a, __fmul_rn(w0, b)));
+}
+
 // Adds a plane's w and v to the moments of an axis.
 __device__ __forceinline__ void add_moments(float (&m)[5], float wv, float vv, float zf) {
-  m[0] += wv;
-  m[1] += wv * zf;
-  m[2] += wv * zf * zf;
-  m[3] += vv;
-  m[4] += vv * zf;
+  const float wz = __fmul_rn(wv, zf);
+  m[0] = __fadd_rn(m[0], wv);
+  m[1] = __fadd_rn(m[1], wz);
+  m[2] = fmaf(wz, zf, m[2]);
+  m[3] = __fadd_rn(m[3], vv);
+  m[4] = fmaf(vv, zf, m[4]);
 }
 
 // SPLIT: a cluster of np CTAs shares a slab, gs planes each.  The CTAs keep the
 // w and v of their planes in shared memory and the first one adds them all
 // plane by plane, so that the FP32 moments are those of one CTA walking the
 // slab, bit for bit, and a volume's result does not depend on the batch it is
-// in.
+// in.  Every rounding on the way from the responses to the sums is written
+// out (which products fuse with an addition is the compiler's choice
+// otherwise, in each form of the kernel for itself).
 template <bool SMOOTH, bool SPLIT>
 __global__ void __launch_bounds__(kMarchWarps * 32, 2)
 normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const float2* __restrict__ q2, int W,
@@ -346,7 +367,7 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
         phase_diff_cert(nw.a[k], nw.c[k], pd, cv);
         cv = cin ? cv : 0.f;
         const float cl = __shfl_up_sync(0xffffffffu, cv, 1), cr = __shfl_down_sync(0xffffffffu, cv, 1);
-        sxr[warp][k][lane] = w1 * cl + w0 * cv + w1 * cr;
+        sxr[warp][k][lane] = smooth3(w0, w1, cl, cv, cr);
       }
     }
     qy1[j][warp][lane] = nw.a[1];
@@ -362,7 +383,7 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
 #pragma unroll
       for (int k = 0; k < 3; k++)
         cxr[SMOOTH ? j : 0][warp][k][lane] =
-            w1 * sxr[warp - 1][k][lane] + w0 * sxr[warp][k][lane] + w1 * sxr[warp + 1][k][lane];
+            smooth3(w0, w1, sxr[warp - 1][k][lane], sxr[warp][k][lane], sxr[warp + 1][k][lane]);
     }
     // [C] sums of output plane z = p - 1
     if (p >= z0 + 1) {
@@ -387,13 +408,13 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
         for (int k = 0; k < 3; k++) {
           float pd, cert;
           phase_diff_cert(cur.a[k], cur.c[k], pd, cert);
-          const float g = phase_grad(ap[k], cur.a[k], am[k], cp[k], cur.c[k], cm[k]);
+          const float g = phase_grad_rn(ap[k], cur.a[k], am[k], cp[k], cur.c[k], cm[k]);
           if (SMOOTH)
-            cert = w1 * cxr[SMOOTH ? j2 : 0][warp][k][lane] + w0 * cxr[SMOOTH ? j1 : 0][warp][k][lane] +
-                   w1 * cxr[SMOOTH ? j : 0][warp][k][lane];  // planes z - 1, z, z + 1
-          const float cg = cert * g;
-          const float wv = cg * g;
-          const float vv = cg * pd;
+            cert = smooth3(w0, w1, cxr[SMOOTH ? j2 : 0][warp][k][lane], cxr[SMOOTH ? j1 : 0][warp][k][lane],
+                           cxr[SMOOTH ? j : 0][warp][k][lane]);  // planes z - 1, z, z + 1
+          const float cg = __fmul_rn(cert, g);
+          const float wv = __fmul_rn(cg, g);
+          const float vv = __fmul_rn(cg, pd);
           if (SPLIT) {
             float* t = s_wv + ((z - z0) * 6 + 2 * k) * kMarchThreads + threadIdx.x;
             t[0] = wv;
@@ -482,7 +503,7 @@ normal_eq_march_kernel(const float2* __restrict__ q1, long long q1_stride, const
 #pragma unroll
     for (int w = 1; w <= 8; w++) {
       const double yd = (double)(3 + yt * 8 - 1 + w) - 0.5 * (double)(H - 1);
-      v += s_part[w][q] * (py == 0 ? 1.0 : (py == 1 ? yd : yd * yd));
+      v = fma(s_part[w][q], py == 0 ? 1.0 : (py == 1 ? yd : yd * yd), v);
     }
     partials[((long long)b * nbx + bx) * kNSums + threadIdx.x] = v;
   }

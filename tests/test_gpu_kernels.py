@@ -161,6 +161,27 @@ def test_warp_field_lanes_of_a_warp_mixed(ctx, shape, far):
     assert torch.equal(m.nan_to_num(), want.nan_to_num())
 
 
+@pytest.mark.parametrize("shape", [(1, 100, 65), (25, 17, 31), (33, 40, 64), (8, 30, 65)])
+def test_warp_affine_batch_size_does_not_change_a_volume(ctx, shape):
+    """A volume warped alone (one plane per thread) and among 200 (two planes)
+    gives the same bits: positions inside, across the edges, far outside,
+    infinite and NaN."""
+    D, H, W = shape
+    tiles = ((W + 31) // 32) * ((H + 7) // 8) * ((D + 1) // 2)
+    assert tiles < 4 * 148 <= tiles * 16  # the launches take both forms
+    g = torch.Generator().manual_seed(D)
+    vol = torch.randn((8,) + shape, generator=g).cuda()
+    p = torch.randn((8, 12), generator=g) * 0.05
+    p[:, :3] *= 40.0
+    p[4, 3], p[5, 1], p[6, 8], p[7, 2] = 2e5, 7e6, float("inf"), float("nan")
+    p = p.cuda()
+    many = ctx.warp_affine(vol.repeat(25, 1, 1, 1), p.repeat(25, 1))
+    for k in range(8):
+        one, all_k = ctx.warp_affine(vol[k:k + 1], p[k:k + 1]), many[k::8]
+        assert torch.equal(all_k.isnan(), one.expand_as(all_k).isnan())
+        assert torch.equal(all_k.nan_to_num(), one.expand_as(all_k).nan_to_num())
+
+
 @pytest.mark.parametrize("batch", [1, 3])
 def test_warp_affine_lanes_of_a_warp_mixed(ctx, batch):
     """A stretch of 2^23 along x about a central voxel: in every warp the lane

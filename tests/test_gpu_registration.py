@@ -216,4 +216,21 @@ def test_batch_size_does_not_change_a_registration(ctx, lin_filters, depth, sigm
         one = ctx.register_linear(ref, four[k:k + 1], lin_filters, 2, certainty_sigma=sigma)
         for name in ("params", "aligned"):
             a, b = many[name][k::4], one[name]
+            assert torch.equal(a.isnan(), b.expand_as(a).isnan())
+            assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b.expand_as(a)))
+
+
+@pytest.mark.parametrize("precision", [L.PREC_TF32, L.PREC_BF16X3])
+def test_batch_size_does_not_change_a_tensor_core_registration(ctx, lin_filters, precision):
+    """As above on the tensor cores, at a size whose resampling takes one plane
+    per thread alone and two among many."""
+    rng = np.random.default_rng(3)
+    ref = cuda(rng.standard_normal((20, 33, 40)) * 100)
+    four = cuda(rng.standard_normal((4, 20, 33, 40)) * 100)
+    many = ctx.register_linear(ref, four.repeat(32, 1, 1, 1), lin_filters, 2, precision=precision, certainty_sigma=1.0)
+    for k in range(4):
+        one = ctx.register_linear(ref, four[k:k + 1], lin_filters, 2, precision=precision, certainty_sigma=1.0)
+        for name in ("params", "aligned"):
+            a, b = many[name][k::4], one[name]
+            assert torch.equal(a.isnan(), b.expand_as(a).isnan())
             assert torch.equal(torch.nan_to_num(a), torch.nan_to_num(b.expand_as(a)))
