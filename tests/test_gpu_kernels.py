@@ -305,3 +305,43 @@ def test_filter_shape_inside_a_capture(lin_filters):
             got = {batch: c.selftest_filter_shape(shape, batch, lin_filters) for batch in queries}
         assert got == queries
     c.close()
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (3, 5, 2), (7, 9, 4), (5, 17, 33), (9, 8, 36), (11, 20, 63)])
+@pytest.mark.parametrize("nf", [3, 6])
+@pytest.mark.parametrize("kind", ["symmetric", "general", "asymmetric"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_filter_launch_shapes_agree(ctx, bank, shape, nf, kind, offset):
+    """Every launch shape of the FP32 filtering that the timing can pick, on
+    widths below and off the quad, depths below the block's and volumes that
+    are not 16-byte aligned: the same responses bit for bit, with nothing
+    written outside them, and within the suite's 1e-4 of the FP64 convolution
+    (the shape of the summation order that all share)."""
+    gen = torch.Generator().manual_seed(sum(shape) + nf)
+    flt = bank["linear" if nf == 3 else "nonlinear"]
+    if kind == "asymmetric":
+        flt = torch.randn((nf, 2, 7, 7, 7), generator=gen).numpy()
+    prec = L.PREC_FP32_GENERAL if kind == "general" else L.PREC_FP32
+    D, H, W = shape
+    vols = torch.randn((2,) + shape, generator=gen)
+    ref = torch.nn.functional.conv3d(vols.double()[:, None], torch.from_numpy(flt).double().flip(2, 3, 4).reshape(
+        2 * nf, 1, 7, 7, 7), padding=3).reshape((2, nf, 2) + shape).movedim(2, -1)
+    src = torch.zeros(vols.numel() + 1, device="cuda")[offset:offset + vols.numel()]
+    src.copy_(vols.reshape(-1))
+    f = np.ascontiguousarray(flt, np.float32)
+    outs = {}
+    for code in range(1, 64):
+        try:
+            ctx.selftest_filter_shape(shape, 2, flt, prec, set=code)
+        except L.BrcError as e:
+            assert e.status == L.BRC_ERR_INVALID
+            continue
+        buf = torch.full((ref.numel() + 64,), 7.0, device="cuda")
+        assert L.lib().brc_filter3d(ctx.handle, src.data_ptr(), W, H, D, 2, W * H * D, f.ctypes.data, nf, prec,
+                                    buf.data_ptr() + 128) == 0
+        assert bool((buf[:32] == 7.0).all()) and bool((buf[-32:] == 7.0).all())
+        outs[code] = buf[32:-32].reshape(ref.shape).cpu()
+    assert len(outs) == (7 if nf == 3 else 5)
+    first = next(iter(outs.values()))
+    assert all(torch.equal(o, first) for o in outs.values())
+    assert float((first.double() - ref).abs().max() / ref.abs().max()) < TOL
