@@ -293,7 +293,6 @@ int make_filter_path(brc_ctx* ctx, const float* h_filters, int nfilt, int precis
                      int batch, FilterPath* fp) {
   if (nfilt != 3 && nfilt != 6) return ctx->fail(BRC_ERR_INVALID, "filtering needs 3 or 6 filters");
   fp->precision = precision;
-  fp->h_filters = h_filters;
   fp->nfilt = nfilt;
   fp->d_taps = nullptr;
   fp->d_err = ctx->tc_err.as<int>();

@@ -158,7 +158,6 @@ struct brc_ctx {
 // tensor-core path).
 struct FilterPath {
   int precision = 0;
-  const float* h_filters = nullptr;
   int nfilt = 3;
   const uint16_t* d_taps = nullptr;
   brc::tc::Geometry g{};

@@ -1090,6 +1090,7 @@ constexpr int kSmYPlane = kSmTY * kSmPY, kSmRPlane = kSmTY * kSmPR;
 constexpr int kSmRGroup = kSmG * kSmRPlane;
 constexpr size_t kSmSmem = sizeof(float) * (kSmG * kSmYPlane + 2 * kSmRGroup);
 static_assert(kSmTY == 8 && kSmG == 8, "the unit decodes assume 8 rows and groups of 8 planes");
+static_assert(kSmSmem <= 48 * 1024, "more needs a function attribute on every device");
 
 // The taps of the three passes, each twice (both lanes of a packed FMA), in
 // the order of the samples (o = -4..4 meets taps 8..0).
@@ -1616,10 +1617,6 @@ cudaError_t smooth3d(const float* vol, int W, int H, int D, int batch, const flo
   const int tw = smooth_tile_width(W);
   const int zc = zchunk > 0 ? (zchunk < D ? zchunk : D) : smooth_chunk(D, ntiles * batch);
   const dim3 grid((unsigned)ntiles, (unsigned)((D + zc - 1) / zc), (unsigned)batch);
-  // the dynamic shared memory above 48 KB is a per-device function attribute
-  static bool attr_set[64] = {false};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
   // 8-byte accesses need an even W (pairs never straddle the edge) and 8-byte
   // aligned volumes
   const bool pairs = (W & 1) == 0 &&
@@ -1628,14 +1625,6 @@ cudaError_t smooth3d(const float* vol, int W, int H, int D, int batch, const flo
   const bool acc = !alias && accumulate != 0;
   const int variant = times_cert ? 16 + (pairs ? 1 : 0)
                                  : (cert ? 8 : 0) | (pairs ? 4 : 0) | (scert ? 2 : 0) | (acc ? 1 : 0);
-  if (!attr_set[dev]) {
-    for (int v = 0; v < 18; v++) {
-      const cudaError_t e0 =
-          cudaFuncSetAttribute(smooth_kernel_of(v), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmSmem);
-      if (e0 != cudaSuccess) return e0;
-    }
-    attr_set[dev] = true;
-  }
   void* args[] = {(void*)&vol, (void*)&cert, (void*)&scert, (void*)&W, (void*)&H,
                   (void*)&D,   (void*)&tw,   (void*)&zc,    (void*)&taps, (void*)&dst};
   {
