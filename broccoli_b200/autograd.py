@@ -22,6 +22,7 @@ graph together.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -46,13 +47,22 @@ def _ctx(device: torch.device) -> Context:
 
 
 _P, _I, _Z = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
+_functions = {}
 
 
 def _sig(name, args, res=_I):
-    fn = getattr(L.lib(), name)
-    fn.argtypes = args
-    fn.restype = res
+    fn = _functions.get(name)
+    if fn is None:
+        fn = getattr(L.lib(), name)
+        fn.argtypes = args
+        fn.restype = res
+        _functions[name] = fn
     return fn
+
+
+@functools.lru_cache(maxsize=1024)
+def _scratch_bytes(name, *sizes):
+    return _sig(name, [_I] * len(sizes), _Z)(*sizes)
 
 
 def gaussian_taps(sigma: float) -> np.ndarray:
@@ -96,7 +106,7 @@ class WarpAffine(torch.autograd.Function):
         B, D, H, W = (s.shape if s.dim() == 4 else (1,) + tuple(s.shape))
         gp = torch.empty((B, 12), dtype=torch.float64, device=g.device)
         gs = torch.empty((B, D, H, W), dtype=torch.float32, device=g.device) if fctx.needs_input_grad[0] else None
-        size = _sig("brc_warp_affine_backward_scratch_bytes", [_I] * 4, _Z)(W, H, D, B)
+        size = _scratch_bytes("brc_warp_affine_backward_scratch_bytes", W, H, D, B)
         sums = torch.empty(size, dtype=torch.uint8, device=g.device)
         fn = _sig("brc_warp_affine_backward_scratch", [_P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _Z])
         _check(c, fn(c.handle, _p(s), W, H, D, B, _p(p), _p(g.contiguous()), _p(gp),
@@ -144,7 +154,7 @@ class Filter3d(torch.autograd.Function):
         B, nf, D, H, W, _ = g.shape
         out = torch.empty((B, D, H, W), dtype=torch.float32, device=g.device)
         fn = _sig("brc_filter3d_adjoint", [_P, _P, _I, _I, _I, _I, _P, _I, _P])
-        _check(c, fn(c.handle, _p(g.contiguous()), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), nf, _p(out)))
+        _check(c, fn(c.handle, _p(g.contiguous()), W, H, D, B, f.ctypes.data, nf, _p(out)))
         return out, None
 
 
@@ -161,17 +171,17 @@ class FilterSsd(torch.autograd.Function):
         B, D, H, W = v.shape
         if not isinstance(q_ref, torch.Tensor) or q_ref.dtype != torch.float32 or q_ref.device != v.device:
             raise TypeError("reference responses must be float32 tensors on the volumes' device")
-        if tuple(q_ref.shape) != (B, f.shape[0], D, H, W, 2):
+        if q_ref.shape != (B, f.shape[0], D, H, W, 2):
             raise ValueError("reference responses must have shape (B, nfilt, D, H, W, 2)")
         c = _ctx(v.device)
         r = q_ref.detach().contiguous()
         res = torch.empty_like(r)
         loss = torch.empty((), dtype=torch.float32, device=v.device)
         # the block sums are torch's memory (as the rows of WarpAffine.backward)
-        size = _sig("brc_filter3d_ssd_scratch_bytes", [_I] * 5, _Z)(W, H, D, B, f.shape[0])
+        size = _scratch_bytes("brc_filter3d_ssd_scratch_bytes", W, H, D, B, f.shape[0])
         sums = torch.empty(size, dtype=torch.uint8, device=v.device)
         fn = _sig("brc_filter3d_ssd_scratch", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _Z])
-        _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), f.shape[0], _p(r), _p(res),
+        _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data, f.shape[0], _p(r), _p(res),
                      _p(loss), _p(sums), size))
         fctx.filters = f
         fctx.vol_shape = vol.shape
@@ -179,8 +189,12 @@ class FilterSsd(torch.autograd.Function):
         return loss
 
     @staticmethod
-    @once_differentiable
     def backward(fctx, g):
+        # gradients of gradients raise (only create_graph can ask for them)
+        return (FilterSsd._gradients_once if torch.is_grad_enabled() else FilterSsd._gradients)(fctx, g)
+
+    @staticmethod
+    def _gradients(fctx, g):
         # saved-tensor hooks may give the residual back in another layout or type
         res, = fctx.saved_tensors
         if res.device != g.device:
@@ -194,8 +208,10 @@ class FilterSsd(torch.autograd.Function):
         if fctx.needs_input_grad[0]:
             gv = torch.empty(fctx.vol_shape, dtype=torch.float32, device=res.device)
             fn = _sig("brc_filter3d_ssd_adjoint", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P])
-            _check(c, fn(c.handle, _p(res), W, H, D, B, f.ctypes.data_as(ctypes.c_void_p), nf, _p(gl), _p(gv)))
+            _check(c, fn(c.handle, _p(res), W, H, D, B, f.ctypes.data, nf, _p(gl), _p(gv)))
         return gv, None, (-2.0 * gl) * res if fctx.needs_input_grad[2] else None
+
+    _gradients_once = staticmethod(once_differentiable(_gradients.__func__))
 
 
 def smooth3d(vol, sigma: float):
@@ -245,5 +261,5 @@ def _fusable(q_ref, w: torch.Tensor, nfilt: int) -> bool:
     goes through torch."""
     return (type(q_ref) in (torch.Tensor, torch.nn.Parameter) and q_ref.layout == torch.strided
             and q_ref.dtype == torch.float32 and q_ref.device == w.device
-            and tuple(q_ref.shape) == (w.shape[0], nfilt) + tuple(w.shape[1:]) + (2,)
+            and q_ref.shape == (w.shape[0], nfilt, *w.shape[1:], 2)
             and not (q_ref.requires_grad and torch.is_grad_enabled()) and unpack_dual(q_ref).tangent is None)
