@@ -187,7 +187,7 @@ class Context:
         sc = smoothed_cert.contiguous() if smoothed_cert is not None else None
         self._bind_stream()
         _check(self, L.lib().brc_smooth3d(self.handle, _p(v), W, H, D, B,
-                                          *[t.ctypes.data_as(ctypes.c_void_p) for t in taps],
+                                          *[t.ctypes.data for t in taps],
                                           _p(c) if c is not None else None,
                                           _p(sc) if sc is not None else None, _p(out)))
         return out if vol.dim() == 4 else out[0]

@@ -102,6 +102,7 @@ class WarpAffine(torch.autograd.Function):
     @staticmethod
     def backward(fctx, g):
         s, p = fctx.saved_tensors
+        g = g.contiguous()
         c = _ctx(g.device)
         B, D, H, W = (s.shape if s.dim() == 4 else (1,) + tuple(s.shape))
         gp = torch.empty((B, 12), dtype=torch.float64, device=g.device)
@@ -109,8 +110,8 @@ class WarpAffine(torch.autograd.Function):
         size = _scratch_bytes("brc_warp_affine_backward_scratch_bytes", W, H, D, B)
         sums = torch.empty(size, dtype=torch.uint8, device=g.device)
         fn = _sig("brc_warp_affine_backward_scratch", [_P, _P, _I, _I, _I, _I, _P, _P, _P, _P, _P, _Z])
-        _check(c, fn(c.handle, _p(s), W, H, D, B, _p(p), _p(g.contiguous()), _p(gp),
-                     _p(gs) if gs is not None else None, _p(sums), size))
+        _check(c, fn(c.handle, s.data_ptr(), W, H, D, B, p.data_ptr(), g.data_ptr(), gp.data_ptr(),
+                     gs.data_ptr() if gs is not None else None, sums.data_ptr(), size))
         gsrc = gs.reshape(s.shape) if gs is not None else None
         return gsrc, gp.to(torch.float32).reshape(fctx.saved_tensors[1].shape)
 
@@ -181,8 +182,8 @@ class FilterSsd(torch.autograd.Function):
         size = _scratch_bytes("brc_filter3d_ssd_scratch_bytes", W, H, D, B, f.shape[0])
         sums = torch.empty(size, dtype=torch.uint8, device=v.device)
         fn = _sig("brc_filter3d_ssd_scratch", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P, _P, _P, _Z])
-        _check(c, fn(c.handle, _p(v), W, H, D, B, f.ctypes.data, f.shape[0], _p(r), _p(res),
-                     _p(loss), _p(sums), size))
+        _check(c, fn(c.handle, v.data_ptr(), W, H, D, B, f.ctypes.data, f.shape[0], r.data_ptr(), res.data_ptr(),
+                     loss.data_ptr(), sums.data_ptr(), size))
         fctx.filters = f
         fctx.vol_shape = vol.shape
         fctx.save_for_backward(res)
@@ -199,7 +200,8 @@ class FilterSsd(torch.autograd.Function):
         res, = fctx.saved_tensors
         if res.device != g.device:
             raise TypeError("the saved residual must be on the gradient's device")
-        res = res.to(torch.float32).contiguous()
+        if res.dtype != torch.float32 or not res.is_contiguous():
+            res = res.to(torch.float32).contiguous()
         c = _ctx(res.device)
         f = fctx.filters
         B, nf, D, H, W, _ = res.shape
@@ -208,7 +210,7 @@ class FilterSsd(torch.autograd.Function):
         if fctx.needs_input_grad[0]:
             gv = torch.empty(fctx.vol_shape, dtype=torch.float32, device=res.device)
             fn = _sig("brc_filter3d_ssd_adjoint", [_P, _P, _I, _I, _I, _I, _P, _I, _P, _P])
-            _check(c, fn(c.handle, _p(res), W, H, D, B, f.ctypes.data, nf, _p(gl), _p(gv)))
+            _check(c, fn(c.handle, res.data_ptr(), W, H, D, B, f.ctypes.data, nf, gl.data_ptr(), gv.data_ptr()))
         return gv, None, (-2.0 * gl) * res if fctx.needs_input_grad[2] else None
 
     _gradients_once = staticmethod(once_differentiable(_gradients.__func__))
