@@ -55,3 +55,18 @@ def test_default_options():
     L.lib().brc_linear_opts_default(ctypes.byref(o), 20)
     assert (o.iterations, o.type, o.precision, o.use_graph, o.certainty_sigma_x100) == (20, L.AFFINE, 0, 1, 0)
     assert o.tolerance == 0.0
+
+
+@pytest.mark.parametrize("name, sizes, largest", [
+    ("brc_filter3d_ssd_scratch_bytes", (128, 128, 96, 2, 3), 148 * 8 * 8),
+    ("brc_warp_affine_backward_scratch_bytes", (128, 128, 96, 2), 148 * 4 * 12 * 2 * 8)])
+def test_scratch_sizes(name, sizes, largest):
+    """A positive multiple of eight up to the full grid's sums; 0 for sizes that
+    the entry point refuses."""
+    fn = getattr(L.lib(), name)
+    fn.argtypes, fn.restype = [ctypes.c_int] * len(sizes), ctypes.c_size_t
+    assert fn(*sizes) == largest
+    assert 0 < fn(*(1,) * 4 + sizes[4:]) <= largest and fn(*(1,) * 4 + sizes[4:]) % 8 == 0
+    for i in range(len(sizes)):
+        for bad in (0, -1):
+            assert fn(*sizes[:i] + (bad,) + sizes[i + 1:]) == 0
