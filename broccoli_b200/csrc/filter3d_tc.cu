@@ -405,9 +405,9 @@ filter3d_tc_kernel(const float* __restrict__ vol, const uint16_t* __restrict__ t
     // loads of the next tile's first rows are issued before this thread waits
     // for that tile's buffer.  (199 volumes of 64x64x33: 375 -> 357 us; six
     // filters at 182x218x182, whose rows are not 16-byte aligned and were
-    // loaded one sample at a time: 173 -> 168 us.  Neither is bound by one
-    // role now: without the staging's loads, the stores, the tap copies or with
-    // N = 16 the launch takes 80-87 % of its time.)
+    // loaded one sample at a time: 173 -> 168 us.  The 199 volumes are not
+    // bound by one role now: without the stores, with small tap copies or with
+    // N = 16 the launch takes 86-88 % of its time.)
     const int st = tid - kStageWarp * 32;
     const int nit = (nrows + kStageThreads - 1) / kStageThreads;
     const float* const vbeg = vol;

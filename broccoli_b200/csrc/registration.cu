@@ -957,10 +957,11 @@ __global__ void solve_given_kernel(const double* __restrict__ A, const double* _
 // instructions per warp and voxel row; LSU 44 %, DRAM 8 %).  A thread takes the same
 // voxel of two planes: the instance's part and the x and y terms once, the
 // positions and interpolations as packed pairs.  One plane to two, us:
-// 199 x 64x64x33 135.0 -> 123.8-125.2, 59 x 80x80x37 88.3 -> 78.1, 24 x 64x64x33
-// 22.9 -> 19.1, one 182x218x182 53.5 -> 39.2.  56 registers, four blocks per SM; five and six blocks are slower
-// (130.6 and 139.5 us at the first size), as is clamping x alone where y and z
-// are inside (121.8 us there, but 43.3 at 182x218x182).
+// 199 x 64x64x33 135.0 -> 123.2-125.0, 59 x 80x80x37 88.3 -> 77.5-77.9, 24 x
+// 64x64x33 22.9 -> 18.7, one 182x218x182 53.5 -> 39.2.  56 registers, four blocks
+// per SM; five and six blocks are slower (130.6 and 139.5 us at the first size),
+// as is clamping x alone where y and z are inside (121.8 us there, but 43.3 at
+// 182x218x182).
 template <bool VEC, int NZ>
 __global__ void __launch_bounds__(256)
 warp_affine_kernel(const float* __restrict__ src, long long src_stride, int W, int H, int D, int ntx, int batch,
@@ -1074,7 +1075,9 @@ rescale_linear_kernel(const float* __restrict__ src, int W, int H, int D, float*
 // plane and a register ring for z issued 109 thread instructions per voxel
 // for its 27 FMAs.  Packed FP32 FMAs (two lanes per instruction, rounded as
 // two scalar ones) halve the issue slots of the arithmetic.
-// Measured (CUDA events): 9 volumes of 182x218x182 278 -> 169 us (3.1 TB/s),
+// Measured (CUDA events, passes back to back): 9 volumes of 182x218x182 278 ->
+// 168 us (3.1 TB/s; 172-174 with the inputs of several passes in turn, 188 for a
+// pass that starts on an idle GPU),
 // 9 of 91x109x91 (odd width) 59 -> 36 us, 200 of 64x64x33 175 -> 73 us (3.0
 // TB/s), the same with certainty, division and mask product in the kernel
 // 360 -> 160 us.  Tiles of 64 columns with 288 threads: 174, 37, 73, 173 us
@@ -1109,8 +1112,9 @@ __host__ __device__ inline int smooth_tile_width(int W) {
 // and 8-byte aligned volumes); DIV: divide by the smoothed certainty scert;
 // MUL: then multiply by the certainty; ACC: add into `out`.
 template <bool CERT, bool VEC, bool DIV, bool MUL, bool ACC>
-// Five blocks per SM where pairs move and there is no certainty; the other
-// forms spill there (certainty 194 against 160 us with four).
+// Five blocks per SM where pairs move and there is no certainty (of these the two
+// that divide spill 12 bytes); the certainty forms take four (194 us with five,
+// 160 with four), and so do single accesses.
 __global__ void __launch_bounds__(kSmThreads, VEC && !CERT ? 5 : 4)
 smooth3d_kernel(const float* __restrict__ in, const float* __restrict__ cert, const float* __restrict__ scert,
                 int W, int H, int D, int tw, int zc, const __grid_constant__ SmoothTaps taps,
